@@ -157,10 +157,11 @@ extern "C" int chb_dot(chb_plan* plan, const double* x, const double* y, double*
   clear_error();
   int rc = check_plan(plan);
   if (rc) return rc;
-  const size_t need = 256 + (size_t)(plan->nsn + 1) * sizeof(double);
+  const size_t need = 256 + (size_t)(plan->npieces + 1) * sizeof(double);
   if (work_bytes < need || !work) return set_error(-4, "workspace too small: %zu bytes given, %zu needed", work_bytes, need);
   double* partial = (double*)((char*)work + 256);
-  cudaError_t e = dot_launch(x, y, plan->d_fronts, (int)plan->nsn, partial, result, (cudaStream_t)stream);
+  cudaError_t e = dot_launch(x, y, plan->d_fronts, plan->d_red, (int)plan->npieces, partial, result,
+                             (cudaStream_t)stream);
   if (e != cudaSuccess) return set_error(-100 - (int)e, "dot launch failed: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -185,13 +186,13 @@ static int batch_reduce(chb_plan* plan, const double* a, const double* b, bool l
   clear_error();
   int rc = check_plan(plan);
   if (rc) return rc;
-  const size_t need = 256 + (size_t)(plan->nsn + 1) * sizeof(double);
+  const size_t need = 256 + (size_t)((logdet ? plan->nsn : plan->npieces) + 1) * sizeof(double);
   if (work_bytes < need || !work) return set_error(-4, "workspace too small: %zu bytes given, %zu needed", work_bytes, need);
   double* partial = (double*)((char*)work + 256);
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = logdet ? logdet_partials(a, plan->d_fronts, (int)plan->nsn, partial, st)
-                         : dot_partials(a, b, plan->d_fronts, (int)plan->nsn, partial, st);
-  if (e == cudaSuccess) e = segment_sums(partial, plan->d_seg, (int)plan->seg.size() - 1, results, st);
+                         : dot_partials(a, b, plan->d_fronts, plan->d_red, (int)plan->npieces, partial, st);
+  if (e == cudaSuccess) e = segment_sums(partial, logdet ? plan->d_seg : plan->d_red_seg, (int)plan->seg.size() - 1, results, st);
   if (e != cudaSuccess) return set_error(-100 - (int)e, "reduction launch failed: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -219,7 +220,7 @@ extern "C" int chb_sym_weight(chb_plan* plan, const double* x, double* y, double
   clear_error();
   int rc = check_plan(plan);
   if (rc) return rc;
-  cudaError_t e = symw_launch(x, y, alpha, plan->d_fronts, (int)plan->nsn, (cudaStream_t)stream);
+  cudaError_t e = symw_launch(x, y, alpha, plan->d_fronts, plan->d_red, (int)plan->npieces, (cudaStream_t)stream);
   if (e != cudaSuccess) return set_error(-100 - (int)e, "sym_weight launch failed: %s", cudaGetErrorString(e));
   return 0;
 }

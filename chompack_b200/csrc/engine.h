@@ -149,6 +149,16 @@ struct FrontDesc {
   int64_t vpos;         // sum of na over the preceding supernodes (vector updates)
 };
 
+// A piece of the block values for the element-wise reductions (dot,
+// sym_weight): len entries from off, the first one in supernode sn.  A
+// plan's list ends with an empty piece (sn: the last supernode).
+struct RedPiece {
+  int64_t off;
+  int32_t sn;
+  int32_t len;
+};
+constexpr int RED_PIECE = 4096;  // entries of a full piece
+
 // Device-side run description (passed by value to the persistent kernel).
 struct RunArgs {
   const Task* tasks;

@@ -339,8 +339,31 @@ using namespace chb;
 
 // Device copies of the plan's symbolic data (skipped with device < 0: a
 // host-only plan for introspection) and the persistent grid size.
+// The pieces of the block values: at most RED_PIECE entries each, cut at the
+// matrices of a merged plan.
+static std::vector<RedPiece> red_pieces(chb_plan* P) {
+  std::vector<RedPiece> v;
+  P->red_seg.assign(1, 0);
+  for (size_t m = 0; m + 1 < P->seg.size(); m++) {
+    const int64_t k0 = P->seg[m], k1 = P->seg[m + 1];
+    const int64_t beg = k0 < P->nsn ? P->fronts[k0].blk : P->blk_total;
+    const int64_t end = k1 < P->nsn ? P->fronts[k1].blk : P->blk_total;
+    int64_t k = k0;
+    for (int64_t o = beg; o < end; o += RED_PIECE) {
+      while (k + 1 < k1 && P->fronts[k + 1].blk <= o) k++;
+      v.push_back({o, (int32_t)k, (int32_t)std::min<int64_t>(RED_PIECE, end - o)});
+    }
+    P->red_seg.push_back((int64_t)v.size());
+  }
+  P->npieces = (int64_t)v.size();
+  v.push_back({P->blk_total, (int32_t)std::max<int64_t>(P->nsn - 1, 0), 0});
+  return v;
+}
+
 static int upload_plan(chb_plan* P) {
   const int device = P->device;
+  const std::vector<RedPiece> red = red_pieces(P);
+  if (P->npieces > INT32_MAX / 2) return set_error(-7, "block values exceed the reductions' index range");
   if (device < 0) return 0;
   const int64_t nsn = P->nsn, n = P->n, nrel = (int64_t)P->relidx.size();
   CUDA_TRY(cudaSetDevice(device));
@@ -375,6 +398,10 @@ static int upload_plan(chb_plan* P) {
       CUDA_TRY(cudaMemcpy(P->d_symv_items, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice));
     }
   }
+  CUDA_TRY(cudaMalloc(&P->d_red, red.size() * sizeof(RedPiece)));
+  CUDA_TRY(cudaMemcpy(P->d_red, red.data(), red.size() * sizeof(RedPiece), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMalloc(&P->d_red_seg, P->red_seg.size() * sizeof(int64_t)));
+  CUDA_TRY(cudaMemcpy(P->d_red_seg, P->red_seg.data(), P->red_seg.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
   CUDA_TRY(cudaMalloc(&P->d_seg, P->seg.size() * sizeof(int64_t)));
   CUDA_TRY(cudaMemcpy(P->d_seg, P->seg.data(), P->seg.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
   int per_sm = 0, nsm = 0;
@@ -552,6 +579,8 @@ extern "C" int chb_plan_destroy(chb_plan* plan) {
   if (plan->d_perm) cudaFree(plan->d_perm);
   if (plan->d_iperm) cudaFree(plan->d_iperm);
   if (plan->d_seg) cudaFree(plan->d_seg);
+  if (plan->d_red) cudaFree(plan->d_red);
+  if (plan->d_red_seg) cudaFree(plan->d_red_seg);
   if (plan->d_symv_items) cudaFree(plan->d_symv_items);
   delete plan;
   return 0;
@@ -561,8 +590,8 @@ extern "C" int chb_workspace_size(const chb_plan* plan_c, int op, int64_t k, int
   clear_error();
   chb_plan* plan = const_cast<chb_plan*>(plan_c);
   if (!plan || !bytes) return set_error(-1, "null argument");
-  if (op == CHB_OP_DOT) {  // per-supernode partial sums
-    *bytes = 256 + (size_t)(plan->nsn + 1) * sizeof(double);
+  if (op == CHB_OP_DOT) {  // partial sums, one per supernode (log det) or piece (dot)
+    *bytes = 256 + (size_t)(std::max(plan->nsn, plan->npieces) + 1) * sizeof(double);
     return 0;
   }
   Program* p = build_host_program(plan, op, k, flags);

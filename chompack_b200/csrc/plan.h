@@ -108,6 +108,10 @@ struct chb_plan {
   int64_t* d_iperm = nullptr;   // inverse of p (sparse assembly)
   std::vector<int64_t> seg;     // matrices of a merged plan: supernodes [seg[m], seg[m+1])
   int64_t* d_seg = nullptr;
+  std::vector<int64_t> red_seg;   // matrix m: pieces [red_seg[m], red_seg[m+1])
+  int64_t* d_red_seg = nullptr;
+  chb::RedPiece* d_red = nullptr; // pieces of the block values (npieces, then an empty one)
+  int64_t npieces = 0;
   int2* d_symv_items = nullptr;  // 64-row strips of the supernode blocks (supernode, first row)
   int n_symv_items = 0;
   int grid = 0;                 // persistent grid size (the FP64 instantiation)
@@ -165,17 +169,17 @@ cudaError_t engine_launch(const RunArgs& ra, int grid, cudaStream_t stream);
 int engine_occupancy(int* blocks_per_sm, bool tc = false);
 cudaError_t logdet_launch(const double* l, const FrontDesc* fronts, int nsn, double* partial, double* out,
                           cudaStream_t stream);
-cudaError_t symw_launch(const double* x, double* y, double alpha, const FrontDesc* fronts, int nsn,
-                        cudaStream_t stream);
+cudaError_t symw_launch(const double* x, double* y, double alpha, const FrontDesc* fronts, const RedPiece* pieces,
+                        int npieces, cudaStream_t stream);
 cudaError_t segment_sums(const double* partial, const int64_t* seg, int count, double* out, cudaStream_t stream);
 cudaError_t symv_launch(const double* blkval, const FrontDesc* fronts, const int2* items, int nitems,
                         const int64_t* sncolptr, const int64_t* snrowidx, const int64_t* perm, const double* x,
                         double* y, int nrhs, int64_t ld, double alpha, cudaStream_t stream);
 cudaError_t logdet_partials(const double* l, const FrontDesc* fronts, int nsn, double* partial, cudaStream_t stream);
-cudaError_t dot_partials(const double* x, const double* y, const FrontDesc* fronts, int nsn, double* partial,
-                         cudaStream_t stream);
-cudaError_t dot_launch(const double* x, const double* y, const FrontDesc* fronts, int nsn, double* partial,
-                       double* out, cudaStream_t stream);
+cudaError_t dot_partials(const double* x, const double* y, const FrontDesc* fronts, const RedPiece* pieces,
+                         int npieces, double* partial, cudaStream_t stream);
+cudaError_t dot_launch(const double* x, const double* y, const FrontDesc* fronts, const RedPiece* pieces, int npieces,
+                       double* partial, double* out, cudaStream_t stream);
 
 // Program builders (one per sweep), in build_*.cpp.
 int build_cholesky(const chb_plan& P, Program& prog);
