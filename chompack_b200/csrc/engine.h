@@ -1,5 +1,5 @@
 // Task-graph engine shared by the host planner (plan.cpp) and the device
-// executor (engine.cu).
+// executor (engine_kernel.cuh, built by engine.cu, engine_tc.cu, engine_ql.cu).
 //
 // Every numeric sweep is compiled on the host into a list of tile tasks in a
 // topological order.  One persistent kernel executes the list: each CTA
@@ -42,9 +42,25 @@ constexpr int ENGINE_SMEM_DOUBLES = 14336;
 constexpr int TRSV_KMAX = 192;
 constexpr int TRSV_LA = TILE + 2;
 static_assert(TRSV_KMAX * TRSV_LA + TRSV_KMAX * 8 <= ENGINE_SMEM_DOUBLES, "T_TRSV staging exceeds shared memory");
-// Shared-memory doubles a Householder panel of h rows and nb columns needs
-// (panel, then its nb x nb T factor, plus scalars).
-CHB_HD constexpr int ql_panel_doubles(int h, int nb) { return h * nb + nb * nb + 192; }
+// Householder panels of h rows.  Up to QL_REG_ROWS rows a panel is reduced in
+// registers, at most 64 entries a thread, which bounds its columns.
+constexpr int QL_REG_ROWS = 512;
+CHB_HD constexpr int ql_max_cols(int h) { return h <= 128 ? 56 : h <= 256 ? 32 : h <= QL_REG_ROWS ? 12 : 16; }
+// Shared-memory doubles of a panel: the panel (leading dimension ql_ld:
+// congruent to 4 mod 8, so that MMA fragments of eight columns meet no bank
+// twice), its T factor in whole 8 x 8 blocks, a tile per warp, the exchange
+// buffers and the scalars.  A single column needs no T factor and no
+// padding, so the tallest panel has 14,288 rows.
+constexpr int QL_SLD = 12;
+CHB_HD constexpr int ql_ld(int h) { return (h + 3) / 8 * 8 + 4; }
+CHB_HD constexpr int ql_scalars(int nb) { return nb > 1 ? TILE : 8; }
+CHB_HD constexpr int ql_vb_doubles(int h) {  // three reflectors with tau; partial norms and products
+  return h <= 128 ? 396 : h <= 256 ? 780 : h <= QL_REG_ROWS ? 1548 : 32;
+}
+CHB_HD constexpr int ql_panel_doubles(int h, int nb) {
+  return (nb > 1 ? ql_ld(h) * nb + ql_ld((nb + 7) / 8 * 8) * ((nb + 7) / 8 * 8) + NTHREADS / 32 * 8 * QL_SLD : h) +
+         ql_vb_doubles(h) + (h <= QL_REG_ROWS ? 16 * (NTHREADS / 32) : 0) + 2 * ql_scalars(nb);
+}
 
 // Base-pointer slots a task operand refers to.
 enum Base : uint8_t {
@@ -96,6 +112,13 @@ enum TaskOp : uint8_t {
   T_PSUBTREE = 18, // projected_inverse of such ranges, one per warp, parents first
   T_TRSV = 19     // a block-substitution step C = alpha opA opB^T (+ beta C), m <= 64, K <= TRSV_KMAX:
                   // opA (independent of the chain) staged before the mid waits [cdiag, nwait)
+};
+
+// Builds of the persistent kernel.
+enum EngineBuild : int {
+  EB_BASE = 0,     // FP64 and warp-level TF32 sweeps without Householder panels
+  EB_TCGEN05 = 1,  // TF32 tiles on tcgen05
+  EB_PANELS = 2    // programs with T_QL tasks
 };
 
 // Sub-operations of T_QL (child aux[0], columns [aux[1], aux[2]) of the
@@ -184,6 +207,7 @@ struct RunArgs {
   int dynamic;
   int nwords;                     // ready-bitmap words (64 tasks each)
   int nsumm;                      // summary words (64 bitmap words each)
+  int panels;                     // 1: the program has Householder panels (T_QL)
   int tmem;                       // 1: TF32 GEMM tiles run on tcgen05 (tensor memory allocated per CTA)
   int* pend;                      // unmet dependencies per task
   unsigned long long* ready;      // ready, unclaimed tasks

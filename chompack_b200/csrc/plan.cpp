@@ -153,8 +153,10 @@ Program* build_host_program(chb_plan* plan, int op, int64_t k, int flags) {
     for (Task& t : prog->tasks)
       if (t.op == T_GEMM) t.c.prec = prec;
   prog->tf32_tiles = prec == PREC_TF32;
-  for (const Task& t : prog->tasks)
+  for (const Task& t : prog->tasks) {
     if (t.op == T_QL || t.op == T_TRSV) prog->smem_doubles = ENGINE_SMEM_DOUBLES;  // Householder panels, step operands
+    if (t.op == T_QL) prog->panels = true;
+  }
   // Default schedule per sweep, by measurement on a 3-D grid of 64,000
   // unknowns: the chains of small dependent tasks of cholesky, llt and trsm
   // run faster in static list order (a CTA already waits on the next task;
@@ -247,6 +249,7 @@ int run_program(chb_plan* plan, Program* prog, void* work, size_t work_bytes, do
   // TF32 tiles as warp-level mma.sync, or on tcgen05 with tensor-memory
   // accumulators when the plan asks for it
   ra.tmem = prog->tf32_tiles && tf32_tcgen05(*plan) ? 1 : 0;
+  ra.panels = prog->panels ? 1 : 0;
   ra.ldb = run_ldb;
   ra.alpha = run_alpha;
   // The plan's schedule, else CHB_SCHEDULE (static | dynamic), else the

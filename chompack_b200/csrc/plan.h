@@ -37,6 +37,7 @@ struct Program {
   std::vector<int2> waits;
   int64_t ncounters = 0;   // tasks + groups
   int64_t ws_doubles = 0;  // doubles of workspace (update matrices + scratch)
+  bool panels = false;                          // has Householder panels (T_QL tasks)
   int smem_doubles = ENGINE_SMEM_BASE_DOUBLES;  // dynamic shared memory per CTA
   bool static_default = false;  // list order unless the plan asks otherwise
   bool tf32_tiles = false;      // some GEMM tile computes in TF32 (one product)
@@ -163,7 +164,7 @@ constexpr int PF_TF32X3 = 1 << 19;
 int run_program(chb_plan* plan, Program* prog, void* work, size_t work_bytes, double* const* bases, int nbases,
                 cudaStream_t stream, int64_t run_ldb = 0, double run_alpha = 1.0, const HostIo* io = nullptr);
 
-// Device entry points implemented in engine.cu.
+// Device entry points implemented in engine.cu (and the other builds of the kernel).
 size_t engine_smem_bytes();
 cudaError_t engine_launch(const RunArgs& ra, int grid, cudaStream_t stream);
 int engine_occupancy(int* blocks_per_sm, bool tc = false);

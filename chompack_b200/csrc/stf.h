@@ -383,7 +383,9 @@ inline int stf_update_factor(Stf& S, KeyGen& kg, const chb_plan& P, int c, const
       const int row1 = na - N2 + c1 - 1;
       auto h_of = [&](int nb) { return row1 - (r[N1 + c1 - nb] - nn) + 1; };
       int nb = 0;
-      while (nb < c1 - tstart && ql_panel_doubles(h_of(nb + 1), nb + 1) <= ENGINE_SMEM_DOUBLES) nb++;
+      while (nb < c1 - tstart && nb < ql_max_cols(h_of(nb + 1)) &&
+             ql_panel_doubles(h_of(nb + 1), nb + 1) <= ENGINE_SMEM_DOUBLES)
+        nb++;
       if (nb == 0) return set_error(-1, "update_factor: a Householder column of %d rows exceeds shared memory", h_of(1));
       const int c0 = c1 - nb;
       const int row0 = r[N1 + c0] - nn, h = row1 - row0 + 1;
