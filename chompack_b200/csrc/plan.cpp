@@ -157,17 +157,14 @@ Program* build_host_program(chb_plan* plan, int op, int64_t k, int flags) {
     if (t.op == T_QL || t.op == T_TRSV) prog->smem_doubles = ENGINE_SMEM_DOUBLES;  // Householder panels, step operands
     if (t.op == T_QL) prog->panels = true;
   }
-  // Default schedule per sweep, by measurement on a 3-D grid of 64,000
-  // unknowns: the chains of small dependent tasks of cholesky, llt and trsm
-  // run faster in static list order (a CTA already waits on the next task;
-  // trmm has the solve's structure and takes its schedule);
-  // the other sweeps gain from running whichever task is ready.  On a
-  // merged plan (a batch of matrices or value sets) projected_inverse also
-  // runs faster in list order: 256 uneven 2-D grids 36.5 -> 28.0 ms, and the
-  // autotuner picked the static order for both batch workloads of the bench.
-  const bool merged = plan->seg.size() > 2;
-  prog->static_default = op == CHB_OP_CHOLESKY || op == CHB_OP_LLT || op == CHB_OP_TRSM || op == CHB_OP_TRMM ||
-                         op == CHB_OP_CONVENTIONAL || (merged && op == CHB_OP_PROJECTED_INVERSE);
+  // Every sweep runs in static list order by default: a CTA already waits on
+  // its next task, while a task released under the dynamic schedule is
+  // published, found and claimed, about 7 us a hop when the CTAs are idle.
+  // Static against dynamic: unfactored completion on 3-D 40^3 12.5 / 14.0 ms
+  // and on 2-D 60^2 0.58 / 0.88, factored 62.6 / 68.7 and 2.5 / 3.0, full
+  // hessian (unfactored) 31.9 / 35.7 and 1.8 / 2.9, projected_inverse 5.5 /
+  // 5.7 and 0.95 / 1.01, on 2-D 1000^2 9.7 / 12.3, and under a scratch limit
+  // 10.8 / 13.7; no sweep at any measured size was faster dynamically.
   Program* p = prog.get();
   plan->progs[key] = std::move(prog);
   return p;
@@ -252,11 +249,9 @@ int run_program(chb_plan* plan, Program* prog, void* work, size_t work_bytes, do
   ra.panels = prog->panels ? 1 : 0;
   ra.ldb = run_ldb;
   ra.alpha = run_alpha;
-  // The plan's schedule, else CHB_SCHEDULE (static | dynamic), else the
-  // sweep's default.
+  // The plan's schedule, else CHB_SCHEDULE (static | dynamic), else static.
   static const char* sched = std::getenv("CHB_SCHEDULE");
-  bool want_static = prog->static_default;
-  if (sched && std::strcmp(sched, "static") == 0) want_static = true;
+  bool want_static = true;
   if (sched && std::strcmp(sched, "dynamic") == 0) want_static = false;
   if (plan->schedule >= 0) want_static = plan->schedule == 1;
   const bool dynamic = !want_static && prog->d_npend && prog->d_ready0;
