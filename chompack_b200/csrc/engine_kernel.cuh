@@ -1181,9 +1181,8 @@ static __device__ void run_mrow(const RunArgs& ra, const Task& t, const SmemLayo
 // The tile is padded to 64 x 64 with an identity block (which factors and
 // inverts to itself and does not couple to the leading b x b part), then
 // processed in four 16-column blocks J:
-//   (a) the 16x16 diagonal block is factored in registers (lane i holds
-//       row i, right-looking) and inverted (lane c holds column c of
-//       Minv_JJ);
+//   (a) the 16x16 diagonal block is factored and inverted by one warp
+//       (potrf_block16);
 //   (b) panel below: L(r, J) = A(r, J) Minv_JJ^T            (DMMA)
 //   (c) trailing lower triangle: A(r, c) -= L(r, J) L(c, J)^T (DMMA)
 // and the inverse of the whole tile block row by block row:
@@ -1193,16 +1192,19 @@ static __device__ void run_mrow(const RunArgs& ra, const Task& t, const SmemLayo
 // inverts it.  Warps 1-3 meanwhile compute the other panel rows, update the
 // trailing rows below block J (after a named barrier on warp 0's panel
 // rows) and assemble block row J-1 of the inverse.  One block-wide barrier
-// per step; only block row 3 of the inverse follows the last step.
-constexpr int POTRF_LD = TILE + 1;
-// sL, sM, 1 / L(j, j), the pivot-column broadcast (2 x 16), per-warp 16 x 8
-// staging of the inverse assembly (16 x 64 in all)
-constexpr int POTRF_SMEM_DOUBLES = 2 * TILE * POTRF_LD + TILE + 32 + 16 * TILE;
+// per step.  Beside the last block they also form its row's products
+// L(I, :I) M(:I, :I) and store what is final, so that only the product with
+// Minv_II and the last stores follow (they took 10.6k cycles, now 2.2k).
+// (leading dimension of the tiles: with 4 mod 16 the MMA fragments, read
+// along either index, meet no bank twice; TILE + 1 put four lanes on a bank)
+constexpr int POTRF_LD = TILE + 4;
+// sL, sM, an 8 x 8 tile of potrf_block16
+constexpr int POTRF_SMEM_DOUBLES = 2 * TILE * POTRF_LD + 64;
 
 // Phase timing for development builds (-DCHB_PROFILE_POTRF); compiled out
 // otherwise.  Cycles per phase summed over tasks (thread 0's view):
 // diagonal task 0 tile load, 1 panel rows and diagonal-block update,
-// 2 16x16 factor, 3 16x16 inverse, 4 end-of-step barrier, 5 L store,
+// 2 16x16 factor and inverse, 4 end-of-step barrier, 5 L store,
 // 6 last inverse block row, 7 M store, 8 first-part publish; look-ahead
 // 16 mid waits, 17 tile load, 18 L' product, 19 L' store, 20 early signal,
 // 21 L'L'^T product, 22 D update.  Task counts at 12 and 24.
@@ -1231,19 +1233,33 @@ static __device__ unsigned long long g_potrf_phase[32];
   } while (0)
 #endif
 
-// acc += A(16 x K) B(K x 8) with A(r, k) = pa[r + k*lda] and
-// B(k, n) = pb[k*ksb + n*nsb] in shared memory (K a multiple of 4).
+// acc += A(16 x K) B(K x 8) (NEG: -=) with A(r, k) = pa[r + k*lda] and
+// B(k, n) = pb[k*ksb + n*nsb] in shared memory (K a multiple of 8), in two
+// chains of MMAs.
+template <bool NEG>
 __device__ __forceinline__ void warp_mma_16x8(double (&acc)[4], const double* pa, int lda, const double* pb,
-                                              int ksb, int nsb, int K, bool negate) {
+                                              int ksb, int nsb, int K) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  const double sgn = negate ? -1.0 : 1.0;
-#pragma unroll 4
-  for (int k = 0; k < K; k += 4) {
-    const double a0 = sgn * pa[g + (k + q) * lda];
-    const double a1 = sgn * pa[g + 8 + (k + q) * lda];
-    const double b0 = pb[(k + q) * ksb + g * nsb];
-    dmma16(acc, a0, a1, b0);
+  double odd[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+  for (int k = 0; k < K; k += 8) {
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const double a0 = pa[g + (k + 4 * e + q) * lda], a1 = pa[g + 8 + (k + 4 * e + q) * lda];
+      const double b0 = pb[(k + 4 * e + q) * ksb + g * nsb];
+      dmma16(e ? odd : acc, NEG ? -a0 : a0, NEG ? -a1 : a1, b0);
+    }
   }
+#pragma unroll
+  for (int h = 0; h < 4; h++) acc[h] += odd[h];
+}
+
+// FP64 MMA m8n8k4: A 8x4, a = A(g, q); B 4x8, b = B(q, g); C 8x8,
+// c = C(g, 2q + {0, 1}), with g = lane / 4, q = lane % 4.
+__device__ __forceinline__ void dmma8(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
 }
 
 // Named barriers (id 0 is __syncthreads): bar.arrive publishes the
@@ -1262,8 +1278,8 @@ __device__ __forceinline__ void potrf_panel_rows(double* sL, const double* sM, i
   constexpr int LD = POTRF_LD;
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   double a0[4] = {0.0, 0.0, 0.0, 0.0}, a1[4] = {0.0, 0.0, 0.0, 0.0};
-  warp_mma_16x8(a0, sL + jp * LD + r0, LD, sM + jp * LD + jp, LD, 1, 16, false);
-  warp_mma_16x8(a1, sL + jp * LD + r0, LD, sM + jp * LD + jp + 8, LD, 1, 16, false);
+  warp_mma_16x8<false>(a0, sL + jp * LD + r0, LD, sM + jp * LD + jp, LD, 1, 16);
+  warp_mma_16x8<false>(a1, sL + jp * LD + r0, LD, sM + jp * LD + jp + 8, LD, 1, 16);
   __syncwarp();
   const int r = r0 + g, c0 = jp + 2 * q, c1 = c0 + 8;
   sL[c0 * LD + r] = a0[0];
@@ -1284,38 +1300,219 @@ __device__ __forceinline__ void potrf_syrk_tile(double* sL, int jp, int r0, int 
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int r = r0 + g, c = c0 + 2 * q;
   double ac[4] = {sL[c * LD + r], sL[(c + 1) * LD + r], sL[c * LD + r + 8], sL[(c + 1) * LD + r + 8]};
-  warp_mma_16x8(ac, sL + jp * LD + r0, LD, sL + jp * LD + c0, LD, 1, 16, true);
+  warp_mma_16x8<true>(ac, sL + jp * LD + r0, LD, sL + jp * LD + c0, LD, 1, 16);
   if (r >= c) sL[c * LD + r] = ac[0];
   if (r >= c + 1) sL[(c + 1) * LD + r] = ac[1];
   if (r + 8 >= c) sL[c * LD + r + 8] = ac[2];
   if (r + 8 >= c + 1) sL[(c + 1) * LD + r + 8] = ac[3];
 }
 
-// Block row I of the inverse, column tiles tj = first, first + stride, ...
-// of 8 columns: T = L(I, :I) M(:I, :I) (K = 16 I) staged in the warp's own
-// 16x8 area sTw, then M(I, tile) = -Minv_II T.
-__device__ __forceinline__ void potrf_inv_row(const double* sL, double* sM, double* sTw, int I, int first,
-                                              int stride) {
+// Cholesky of the 16 x 16 diagonal block at j0 (factor; else the block
+// already holds L) and its inverse, by one warp, in two 8-column groups.
+// Every lane holds the group's 8 x 8 block and factors it for itself, so the
+// chain from pivot to pivot is rsqrt -> multiply -> FMA with no exchange;
+// beside it lane i reduces row i of the group's columns (the 8 rows of the
+// block, then the 8 rows below) and lane c afterwards forms column c of the
+// block's inverse.  The second diagonal 8 x 8 block takes its rank-8 update,
+// and the block below the inverse's diagonal its two products, by MMAs.
+// One lane per row with every pivot column broadcast through shared memory
+// took 300 cycles a pivot on an idle SM: 19.2k for the 64 of a tile, and 6.4k
+// for its four inverses; this takes 13.8k for both (with library rsqrt()
+// 16.7k), and the whole 64 x 64 task 22k instead of 41.8k cycles.
+// Returns the block's first non-positive pivot (zero pivot when !factor), or
+// -1; such a pivot is taken as 1.
+
+// 1 / sqrt(d) for d in [1e-300, 1e300]: the hardware's approximation (about
+// 20 bits) and one third-order step, y + y e (1/2 + 3/8 e) with
+// e = 1 - d y^2, whose error is about 5/16 e^3.  54 cycles in a dependent
+// chain against 66 for rsqrt(), and no branch.
+__device__ __forceinline__ double rsqrt_normal(double d) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-(d * y), y, 1.0);
+  return fma(fma(e, 0.375, 0.5), y * e, y);
+}
+
+// The pivots of an 8 x 8 block held by every lane (a, lower part), with the
+// lane's row x beside them; r = 1 / L(j, j).  Returns false, with results to
+// be thrown away, when a pivot lies outside [1e-300, 1e300].
+__device__ __forceinline__ bool potrf_pivots8(double (&a)[8][8], double (&x)[8], double (&r)[8]) {
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    // the high words of 1e-300 and 1e300: positive, finite, no NaN between them
+    ok = ok && (unsigned)(__double2hiint(a[j][j]) - 0x01A56E20) < 0x7E37E43Cu - 0x01A56E20u;
+    r[j] = rsqrt_normal(a[j][j]);
+    x[j] *= r[j];
+#pragma unroll
+    for (int i = j + 1; i < 8; i++) a[j][i] *= r[j];
+#pragma unroll
+    for (int c = j + 1; c < 8; c++) {
+#pragma unroll
+      for (int i = c; i < 8; i++) a[c][i] = fma(-a[j][i], a[j][c], a[c][i]);
+      x[c] = fma(-x[j], a[j][c], x[c]);
+    }
+  }
+  return ok;
+}
+
+// The same for any pivots, in place in shared memory (rows b0 .. b0 + nr, a
+// lane each): a non-positive one is taken as 1.  Returns the first, or -1.
+__device__ __forceinline__ int potrf_pivots8_any(double* sL, int b0, int nr) {
   constexpr int LD = POTRF_LD;
-  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  const int i0 = 16 * I, ntj = i0 / 8;
-  for (int tj = first; tj < ntj; tj += stride) {
-    double ac[4] = {0.0, 0.0, 0.0, 0.0};
-    warp_mma_16x8(ac, sL + i0, LD, sM + (8 * tj) * LD, 1, LD, i0, false);
-    const int c = 2 * q;
-    sTw[g + 16 * c] = ac[0];
-    sTw[g + 16 * (c + 1)] = ac[1];
-    sTw[g + 8 + 16 * c] = ac[2];
-    sTw[g + 8 + 16 * (c + 1)] = ac[3];
+  const int lane = threadIdx.x & 31;
+  int bad = -1;
+#pragma unroll 1
+  for (int j = 0; j < 8; j++) {
+    double* const col = sL + (b0 + j) * LD + b0;
+    const double d = col[j];
+    const bool np = !(d > 0.0);
+    if (np && bad < 0) bad = j;
+    const double rs = rsqrt(np ? 1.0 : d), v = lane < nr ? col[lane] * rs : 0.0;
     __syncwarp();
-    double am[4] = {0.0, 0.0, 0.0, 0.0};
-    warp_mma_16x8(am, sM + i0 * LD + i0, LD, sTw, 1, 16, 16, true);
+    if (lane >= j && lane < nr) col[lane] = lane == j && np ? 1.0 : v;
     __syncwarp();
-    const int c0 = 8 * tj + 2 * q, r0 = i0 + g;
-    sM[c0 * LD + r0] = am[0];
-    sM[(c0 + 1) * LD + r0] = am[1];
-    sM[c0 * LD + r0 + 8] = am[2];
-    sM[(c0 + 1) * LD + r0 + 8] = am[3];
+#pragma unroll 1
+    for (int c = j + 1; c < 8; c++)
+      if (lane >= c && lane < nr) sL[(b0 + c) * LD + b0 + lane] = fma(-v, col[c], sL[(b0 + c) * LD + b0 + lane]);
+    __syncwarp();
+  }
+  return bad;
+}
+
+__device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw, int j0, bool factor) {
+  constexpr int LD = POTRF_LD;
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, c8 = lane & 7;
+  int first_bad = -1;
+#pragma unroll 1
+  for (int h = 0; h < 2; h++) {
+    const int b0 = j0 + 8 * h;
+    double a[8][8], r[8];  // a[c][i]: entry (i, c), i >= c
+    // row b0 + (lane mod 16): of the block, or below it (h = 0)
+    const int row = b0 + (h == 0 ? (lane & 15) : c8);
+    double x[8];
+    auto load = [&] {
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+#pragma unroll
+        for (int i = c; i < 8; i++) a[c][i] = sL[(b0 + c) * LD + b0 + i];
+        x[c] = sL[(b0 + c) * LD + row];
+      }
+    };
+    load();
+    if (factor) {
+      const int nr = h == 0 ? 16 : 8;
+      const bool ok = potrf_pivots8(a, x, r);
+      __syncwarp();
+      if (ok) {
+        if (lane < nr) {
+#pragma unroll
+          for (int c = 0; c < 8; c++)
+            if (lane >= c) sL[(b0 + c) * LD + row] = x[c];
+        }
+      } else {
+        const int bad = potrf_pivots8_any(sL, b0, nr);
+        if (bad >= 0 && first_bad < 0) first_bad = 8 * h + bad;
+        load();
+#pragma unroll
+        for (int j = 0; j < 8; j++) r[j] = 1.0 / a[j][j];
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const bool bad = a[j][j] == 0.0;
+        first_bad = (bad && first_bad < 0) ? 8 * h + j : first_bad;
+        r[j] = 1.0 / (bad ? 1.0 : a[j][j]);
+      }
+    }
+    // column c8 of the inverse, right-looking: as soon as M(l, c) is known it
+    // is added into the partial sums of the later rows
+    double m[8], t[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) t[i] = 0.0;
+#pragma unroll
+    for (int l = 0; l < 8; l++) {
+      m[l] = l == c8 ? r[l] : (l > c8 ? -r[l] * t[l] : 0.0);
+#pragma unroll
+      for (int i = l + 1; i < 8; i++) t[i] = fma(a[l][i], m[l], t[i]);
+    }
+    if (lane < 8) {
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if (i >= c8) sM[(b0 + c8) * LD + b0 + i] = m[i];
+    }
+    __syncwarp();
+    if (factor && h == 0) {
+      // the second diagonal block: A(r, c) -= sum_k L(r, k) L(c, k), lower part
+      const int rr = j0 + 8 + g, cc = j0 + 8 + 2 * q;
+      double v[2] = {sL[cc * LD + rr], sL[(cc + 1) * LD + rr]};
+#pragma unroll
+      for (int k = 0; k < 8; k += 4) {
+        const double w = sL[(j0 + k + q) * LD + rr];
+        dmma8(v, -w, w);
+      }
+      if (rr >= cc) sL[cc * LD + rr] = v[0];
+      if (rr >= cc + 1) sL[(cc + 1) * LD + rr] = v[1];
+      __syncwarp();
+    }
+  }
+  // M21 = -M22 (L21 M11)
+  double v[2] = {0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < 8; k += 4)
+    dmma8(v, sL[(j0 + k + q) * LD + j0 + 8 + g], sM[(j0 + g) * LD + j0 + k + q]);
+  sTw[16 * q + g] = v[0];  // column-major
+  sTw[16 * q + 8 + g] = v[1];
+  __syncwarp();
+  v[0] = v[1] = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; k += 4) dmma8(v, -sM[(j0 + 8 + k + q) * LD + j0 + 8 + g], sTw[8 * g + k + q]);
+  sM[(j0 + 2 * q) * LD + j0 + 8 + g] = v[0];
+  sM[(j0 + 2 * q + 1) * LD + j0 + 8 + g] = v[1];
+  return first_bad;
+}
+
+// Block row I of the inverse, column tiles of 8 columns: first the products
+// T = L(I, :I) M(:I, tile) (K = 16 I) in the tile's place in sM, then, once
+// the diagonal block's inverse is there, M(I, tile) = -Minv_II T in place.
+__device__ __forceinline__ void potrf_inv_products(const double* sL, double* sM, int I, int tj) {
+  constexpr int LD = POTRF_LD;
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, i0 = 16 * I;
+  double ac[4] = {0.0, 0.0, 0.0, 0.0};
+  warp_mma_16x8<false>(ac, sL + i0, LD, sM + (8 * tj) * LD, 1, LD, i0);
+  double* d = sM + (8 * tj + 2 * q) * LD + i0 + g;
+  d[0] = ac[0];
+  d[LD] = ac[1];
+  d[8] = ac[2];
+  d[LD + 8] = ac[3];
+}
+__device__ __forceinline__ void potrf_inv_finish(double* sM, int I, int tj) {
+  constexpr int LD = POTRF_LD;
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, i0 = 16 * I;
+  double am[4] = {0.0, 0.0, 0.0, 0.0};
+  warp_mma_16x8<true>(am, sM + i0 * LD + i0, LD, sM + (8 * tj) * LD + i0, 1, LD, 16);
+  __syncwarp();
+  double* d = sM + (8 * tj + 2 * q) * LD + i0 + g;
+  d[0] = am[0];
+  d[LD] = am[1];
+  d[8] = am[2];
+  d[LD + 8] = am[3];
+}
+
+// Columns [c0, c1), rows [r0, b) of a tile in shared memory to global memory
+// (lower: on and below the diagonal), by the warps first, first + 1, ... 3, a
+// column a warp.
+__device__ __forceinline__ void potrf_store(double* __restrict__ X, int64_t ldx, const double* sX, int b, int c0,
+                                            int c1, int r0, bool lower, int first) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < first) return;
+#pragma unroll 4
+  for (int c = c0 + warp - first; c < c1; c += NTHREADS / 32 - first) {
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int r = lane + 32 * e;
+      if (r >= r0 && r < b && (!lower || r >= c)) X[c * ldx + r] = sX[c * POTRF_LD + r];
+    }
   }
 }
 
@@ -1499,9 +1696,7 @@ static __device__ void run_potrf(const RunArgs& ra, const Task& t, double* smem,
   const int LD = POTRF_LD;
   double* sL = smem;               // [col][row], lower; upper part zero
   double* sM = sL + TILE * LD;     // inverse, upper part zero
-  double* rdiag = sM + TILE * LD;  // 1 / L(j,j)
-  double* colb = rdiag + TILE;     // pivot-column broadcast, 2 x 16
-  double* sT = colb + 32;          // per-warp 16 x 8 staging (warp w at 128 w)
+  double* sT = sM + TILE * LD;     // staging of potrf_block16
   double* __restrict__ X = ra.bases[t.a.base] + t.a.off;
   const int lda = t.a.ld;
   const int info_base = t.aux[0];
@@ -1541,87 +1736,15 @@ static __device__ void run_potrf(const RunArgs& ra, const Task& t, double* smem,
       if (panel) {
         potrf_panel_rows(sL, sM, jp, j0);
         if (below) named_bar_arrive(1, NTHREADS);
+        else if (want_inv) named_bar_arrive(3, NTHREADS);  // the last block
         potrf_syrk_tile(sL, jp, j0, j0);
         potrf_syrk_tile(sL, jp, j0, j0 + 8);
         __syncwarp();
       }
       POTRF_STAMP(1);
-      if (!factor) {
-        // invert-only: reciprocals of the diagonal (a zero pivot is singular)
-        const int il = lane & 15;
-        const double d = sL[(j0 + il) * LD + j0 + il];
-        if (lane < 16) {
-          if (d == 0.0 && j0 + il < b) atomicCAS(&ra.ctl[2], 0, info_base + j0 + il + 1);
-          rdiag[j0 + il] = 1.0 / (d == 0.0 ? 1.0 : d);
-        }
-        __syncwarp();
-      }
-      {
-        // (a) factor the 16x16 diagonal block in registers: lane i < 16 row i
-        const int il = lane & 15;
-        if (factor) {
-        double a[16];
-#pragma unroll
-        for (int c = 0; c < 16; c++) a[c] = sL[(j0 + c) * LD + j0 + il];
-        // The pivot column goes to the other lanes through shared memory (one
-        // store per lane, then broadcast loads): fifteen double shuffles per
-        // pivot are throughput-bound and cost 2.5x more on this part.
-        // The next pivot, a(jj+1, jj+1) - l(jj+1, jj)^2, is formed by lane
-        // jj+1 from its own values right after its multiplier, so the chain
-        // from pivot to pivot is shuffle -> rsqrt -> multiply -> FMA and the
-        // broadcast and the other updates run beside it.
-        double dn = a[0];
-        int first_bad = -1;  // first non-positive pivot, reported once after the loop
-#pragma unroll
-        for (int jj = 0; jj < 16; jj++) {
-          const double d = __shfl_sync(0xffffffffu, dn, jj);
-          const bool bad = !(d > 0.0);
-          first_bad = (bad && first_bad < 0) ? jj : first_bad;
-          const double x = bad ? 1.0 : d;
-          const double rs = rsqrt(x);
-          const double l = (il == jj) ? x * rs : a[jj] * rs;
-          a[jj] = (il >= jj) ? l : a[jj];
-          if (jj + 1 < 16) dn = fma(-l, l, a[jj + 1]);
-          if (lane == jj) rdiag[j0 + jj] = rs;
-          if (lane < 16) colb[16 * (jj & 1) + il] = l;
-          __syncwarp();
-#pragma unroll
-          for (int kk = jj + 1; kk < 16; kk++) {
-            const double lkj = colb[16 * (jj & 1) + kk];
-            if (il >= kk) a[kk] = fma(-l, lkj, a[kk]);
-          }
-        }
-        if (lane == 0 && first_bad >= 0 && j0 + first_bad < b) atomicCAS(&ra.ctl[2], 0, info_base + j0 + first_bad + 1);
-        if (lane < 16) {
-#pragma unroll
-          for (int c = 0; c < 16; c++)
-            if (c <= il) sL[(j0 + c) * LD + j0 + il] = a[c];
-        }
-        }
-        __syncwarp();
-        POTRF_STAMP(2);
-        // inverse of the block: lane c < 16 holds column c,
-        // M(r, c) = -rd(r) sum_{l<r} L(r, l) M(l, c) for r > c, M(c, c) = rd(c),
-        // right-looking: as soon as M(l, c) is known it is added into the
-        // partial sums of all later rows, so the dependent chain per row is
-        // one multiply and one FMA (FP64 latency, not the row's dot product)
-        double m[16], sacc[16];
-#pragma unroll
-        for (int r = 0; r < 16; r++) sacc[r] = 0.0;
-#pragma unroll
-        for (int l = 0; l < 16; l++) {
-          const double rd = rdiag[j0 + l];
-          m[l] = (l == il) ? rd : ((l > il) ? -rd * sacc[l] : 0.0);
-#pragma unroll
-          for (int r = l + 1; r < 16; r++) sacc[r] = fma(sL[(j0 + l) * LD + j0 + r], m[l], sacc[r]);
-        }
-        if (lane < 16) {
-#pragma unroll
-          for (int r = 0; r < 16; r++)
-            if (r >= il) sM[(j0 + il) * LD + j0 + r] = m[r];
-        }
-        POTRF_STAMP(3);
-      }
+      const int bad = potrf_block16(sL, sM, sT, j0, factor);
+      if (lane == 0 && bad >= 0 && j0 + bad < b) atomicCAS(&ra.ctl[2], 0, info_base + j0 + bad + 1);
+      POTRF_STAMP(2);
     } else {
       if (below) {
         const int rb = j0 + 16 * warp;  // warps 1, 2: the panel rows below block J
@@ -1634,31 +1757,39 @@ static __device__ void run_potrf(const RunArgs& ra, const Task& t, double* smem,
           if (c0 <= r0 + 15) potrf_syrk_tile(sL, jp, r0, c0);
         }
       }
-      if (want_inv && J >= 2) potrf_inv_row(sL, sM, sT + 128 * warp, J - 1, warp - 1, NTHREADS / 32 - 1);
+      if (want_inv && J >= 2)
+        for (int tj = warp - 1; tj < 2 * (J - 1); tj += NTHREADS / 32 - 1) {
+          potrf_inv_products(sL, sM, J - 1, tj);
+          __syncwarp();
+          potrf_inv_finish(sM, J - 1, tj);
+        }
+      if (J == NJ - 1 && J > 0) {
+        // beside the last block: its row's products, and the stores of what
+        // is final (columns of L before block J - 1, rows of the inverse
+        // before row J)
+        if (want_inv) {
+          named_bar_sync(2, NTHREADS - 32);  // the inverse's rows before J
+          if (factor) named_bar_sync(3, NTHREADS);  // row J of L up to block J - 1 (warp 0)
+          for (int tj = warp - 1; tj < 2 * J; tj += NTHREADS / 32 - 1) potrf_inv_products(sL, sM, J, tj);
+        }
+        if (factor) potrf_store(X, lda, sL, b, 0, jp, 0, true, 1);
+        if (want_inv) potrf_store(Mout, ldm, sM, j0, 0, j0, 0, false, 1);
+      }
     }
     __syncthreads();
     POTRF_STAMP(4);
   }
-  if (factor) {
-#pragma unroll 8
-    for (int s2 = 0; s2 < TILE * TILE / NTHREADS; s2++) {
-      const int idx = tid + s2 * NTHREADS;
-      const int r = idx % TILE, c = idx / TILE;
-      if (r < b && c < b && r >= c) X[(int64_t)c * lda + r] = sL[c * LD + r];
-    }
-  }
+  // the last block row of the inverse, and what is left to store
+  if (want_inv)
+    for (int tj = warp; tj < 2 * (NJ - 1); tj += NTHREADS / 32) potrf_inv_finish(sM, NJ - 1, tj);
+  POTRF_STAMP(6);
+  const int jl = 16 * (NJ - 1);
+  if (factor) potrf_store(X, lda, sL, b, max(jl - 16, 0), b, 0, true, 0);
   POTRF_STAMP(5);
   if (!want_inv) return;
-  // the last block row of the inverse (rows 1 .. NJ-2 were assembled above)
-  if (NJ >= 2) potrf_inv_row(sL, sM, sT + 128 * warp, NJ - 1, warp, NTHREADS / 32);
   __syncthreads();
-  POTRF_STAMP(6);
-#pragma unroll 8
-  for (int s2 = 0; s2 < TILE * TILE / NTHREADS; s2++) {
-    const int idx = tid + s2 * NTHREADS;
-    const int r = idx % TILE, cc = idx / TILE;
-    if (r < b && cc < b) Mout[(int64_t)cc * ldm + r] = sM[cc * LD + r];
-  }
+  potrf_store(Mout, ldm, sM, b, 0, jl, jl, false, 0);
+  potrf_store(Mout, ldm, sM, b, jl, b, 0, false, 0);
   POTRF_STAMP(7);
   if (t.k > 0) {
     // first part done: L_cc and M_cc are stored; the task's own waiters go
@@ -2066,14 +2197,6 @@ static __device__ void run_copy(const RunArgs& ra, const Task& t) {
 }
 
 // ------------------------------------------------------ update_factor
-// FP64 MMA m8n8k4: A 8x4, a = A(g, q); B 4x8, b = B(q, g); C 8x8,
-// c = C(g, 2q + {0, 1}), with g = lane / 4, q = lane % 4.
-__device__ __forceinline__ void dmma8(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-
 // Sums of eight values over the warp: every lane returns the sum of u[c],
 // c = the lane's bits 4, 3, 2 (halving the values kept at each exchange, so
 // nine shuffles instead of forty).
