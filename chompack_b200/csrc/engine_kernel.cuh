@@ -1271,32 +1271,30 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// Panel rows [r0, r0 + 16) of the 16-column block at jp, in place:
-// L(r, jp + n) = sum_k A(r, jp + k) Minv(n, k), both 16x8 halves by the
-// calling warp (sL, sM: [col][row], leading dimension POTRF_LD).
-__device__ __forceinline__ void potrf_panel_rows(double* sL, const double* sM, int jp, int r0) {
-  constexpr int LD = POTRF_LD;
+// Panel rows [r0, r0 + 16) of a 16-column block, in place:
+// L(r, n) = sum_k A(r, k) Minv(n, k), both 16x8 halves by the calling warp
+// (the block's columns at Lc, leading dimension LDL, Minv at Mb, LDM).
+template <int LDL, int LDM>
+__device__ __forceinline__ void potrf_panel_rows(double* Lc, const double* Mb, int r0) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   double a0[4] = {0.0, 0.0, 0.0, 0.0}, a1[4] = {0.0, 0.0, 0.0, 0.0};
-  warp_mma_16x8<false>(a0, sL + jp * LD + r0, LD, sM + jp * LD + jp, LD, 1, 16);
-  warp_mma_16x8<false>(a1, sL + jp * LD + r0, LD, sM + jp * LD + jp + 8, LD, 1, 16);
+  warp_mma_16x8<false>(a0, Lc + r0, LDL, Mb, LDM, 1, 16);
+  warp_mma_16x8<false>(a1, Lc + r0, LDL, Mb + 8, LDM, 1, 16);
   __syncwarp();
-  const int r = r0 + g, c0 = jp + 2 * q, c1 = c0 + 8;
-  sL[c0 * LD + r] = a0[0];
-  sL[(c0 + 1) * LD + r] = a0[1];
-  sL[c0 * LD + r + 8] = a0[2];
-  sL[(c0 + 1) * LD + r + 8] = a0[3];
-  sL[c1 * LD + r] = a1[0];
-  sL[(c1 + 1) * LD + r] = a1[1];
-  sL[c1 * LD + r + 8] = a1[2];
-  sL[(c1 + 1) * LD + r + 8] = a1[3];
+  double* d = Lc + 2 * q * LDL + r0 + g;
+#pragma unroll
+  for (int h = 0; h < 4; h++) {
+    d[(h & 1) * LDL + (h & 2) * 4] = a0[h];
+    d[(8 + (h & 1)) * LDL + (h & 2) * 4] = a1[h];
+  }
   __syncwarp();
 }
 
 // Lower-triangle part of the 16x8 tile at (r0, c0) minus the rank-16
 // product of the panel block at jp: A(r, c) -= sum_k L(r, jp + k) L(c, jp + k).
+template <int LDL>
 __device__ __forceinline__ void potrf_syrk_tile(double* sL, int jp, int r0, int c0) {
-  constexpr int LD = POTRF_LD;
+  constexpr int LD = LDL;
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int r = r0 + g, c = c0 + 2 * q;
   double ac[4] = {sL[c * LD + r], sL[(c + 1) * LD + r], sL[c * LD + r + 8], sL[(c + 1) * LD + r + 8]};
@@ -1307,8 +1305,10 @@ __device__ __forceinline__ void potrf_syrk_tile(double* sL, int jp, int r0, int 
   if (r + 8 >= c + 1) sL[(c + 1) * LD + r + 8] = ac[3];
 }
 
-// Cholesky of the 16 x 16 diagonal block at j0 (factor; else the block
-// already holds L) and its inverse, by one warp, in two 8-column groups.
+// Cholesky of a 16 x 16 diagonal block sL (factor; else the block already
+// holds L) and its inverse sM (lower part written), by one warp, in two
+// 8-column groups (only the first with cols <= 8, where the rest of the
+// block is the identity).
 // Every lane holds the group's 8 x 8 block and factors it for itself, so the
 // chain from pivot to pivot is rsqrt -> multiply -> FMA with no exchange;
 // beside it lane i reduces row i of the group's columns (the 8 rows of the
@@ -1358,8 +1358,8 @@ __device__ __forceinline__ bool potrf_pivots8(double (&a)[8][8], double (&x)[8],
 
 // The same for any pivots, in place in shared memory (rows b0 .. b0 + nr, a
 // lane each): a non-positive one is taken as 1.  Returns the first, or -1.
+template <int LD>
 __device__ __forceinline__ int potrf_pivots8_any(double* sL, int b0, int nr) {
-  constexpr int LD = POTRF_LD;
   const int lane = threadIdx.x & 31;
   int bad = -1;
 #pragma unroll 1
@@ -1380,13 +1380,13 @@ __device__ __forceinline__ int potrf_pivots8_any(double* sL, int b0, int nr) {
   return bad;
 }
 
-__device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw, int j0, bool factor) {
-  constexpr int LD = POTRF_LD;
+template <int LD, int LDM>
+__device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw, bool factor, int cols = 16) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, c8 = lane & 7;
   int first_bad = -1;
 #pragma unroll 1
-  for (int h = 0; h < 2; h++) {
-    const int b0 = j0 + 8 * h;
+  for (int h = 0; h < (cols > 8 ? 2 : 1); h++) {
+    const int b0 = 8 * h;
     double a[8][8], r[8];  // a[c][i]: entry (i, c), i >= c
     // row b0 + (lane mod 16): of the block, or below it (h = 0)
     const int row = b0 + (h == 0 ? (lane & 15) : c8);
@@ -1411,7 +1411,7 @@ __device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw
             if (lane >= c) sL[(b0 + c) * LD + row] = x[c];
         }
       } else {
-        const int bad = potrf_pivots8_any(sL, b0, nr);
+        const int bad = potrf_pivots8_any<LD>(sL, b0, nr);
         if (bad >= 0 && first_bad < 0) first_bad = 8 * h + bad;
         load();
 #pragma unroll
@@ -1439,16 +1439,16 @@ __device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw
     if (lane < 8) {
 #pragma unroll
       for (int i = 0; i < 8; i++)
-        if (i >= c8) sM[(b0 + c8) * LD + b0 + i] = m[i];
+        if (i >= c8) sM[(b0 + c8) * LDM + b0 + i] = m[i];
     }
     __syncwarp();
     if (factor && h == 0) {
       // the second diagonal block: A(r, c) -= sum_k L(r, k) L(c, k), lower part
-      const int rr = j0 + 8 + g, cc = j0 + 8 + 2 * q;
+      const int rr = 8 + g, cc = 8 + 2 * q;
       double v[2] = {sL[cc * LD + rr], sL[(cc + 1) * LD + rr]};
 #pragma unroll
       for (int k = 0; k < 8; k += 4) {
-        const double w = sL[(j0 + k + q) * LD + rr];
+        const double w = sL[(k + q) * LD + rr];
         dmma8(v, -w, w);
       }
       if (rr >= cc) sL[cc * LD + rr] = v[0];
@@ -1456,19 +1456,23 @@ __device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw
       __syncwarp();
     }
   }
+  if (cols <= 8) {  // the second half is the identity, as L's is
+    if (lane < 8) sM[(8 + lane) * LDM + 8 + lane] = 1.0;
+    return first_bad;
+  }
   // M21 = -M22 (L21 M11)
   double v[2] = {0.0, 0.0};
 #pragma unroll
   for (int k = 0; k < 8; k += 4)
-    dmma8(v, sL[(j0 + k + q) * LD + j0 + 8 + g], sM[(j0 + g) * LD + j0 + k + q]);
+    dmma8(v, sL[(k + q) * LD + 8 + g], sM[g * LDM + k + q]);
   sTw[16 * q + g] = v[0];  // column-major
   sTw[16 * q + 8 + g] = v[1];
   __syncwarp();
   v[0] = v[1] = 0.0;
 #pragma unroll
-  for (int k = 0; k < 8; k += 4) dmma8(v, -sM[(j0 + 8 + k + q) * LD + j0 + 8 + g], sTw[8 * g + k + q]);
-  sM[(j0 + 2 * q) * LD + j0 + 8 + g] = v[0];
-  sM[(j0 + 2 * q + 1) * LD + j0 + 8 + g] = v[1];
+  for (int k = 0; k < 8; k += 4) dmma8(v, -sM[(8 + k + q) * LDM + 8 + g], sTw[8 * g + k + q]);
+  sM[2 * q * LDM + 8 + g] = v[0];
+  sM[(2 * q + 1) * LDM + 8 + g] = v[1];
   return first_bad;
 }
 
@@ -1693,7 +1697,7 @@ __device__ __forceinline__ void potrf_lookahead(const RunArgs& ra, const Task& t
 
 static __device__ void run_potrf(const RunArgs& ra, const Task& t, double* smem, int ti) {
   const int b = t.m;
-  const int LD = POTRF_LD;
+  constexpr int LD = POTRF_LD;
   double* sL = smem;               // [col][row], lower; upper part zero
   double* sM = sL + TILE * LD;     // inverse, upper part zero
   double* sT = sM + TILE * LD;     // staging of potrf_block16
@@ -1734,27 +1738,27 @@ static __device__ void run_potrf(const RunArgs& ra, const Task& t, double* smem,
     const bool below = panel && J < NJ - 1; // rows below block J to update
     if (warp == 0) {
       if (panel) {
-        potrf_panel_rows(sL, sM, jp, j0);
+        potrf_panel_rows<LD, LD>(sL + jp * LD, sM + jp * LD + jp, j0);
         if (below) named_bar_arrive(1, NTHREADS);
         else if (want_inv) named_bar_arrive(3, NTHREADS);  // the last block
-        potrf_syrk_tile(sL, jp, j0, j0);
-        potrf_syrk_tile(sL, jp, j0, j0 + 8);
+        potrf_syrk_tile<LD>(sL, jp, j0, j0);
+        potrf_syrk_tile<LD>(sL, jp, j0, j0 + 8);
         __syncwarp();
       }
       POTRF_STAMP(1);
-      const int bad = potrf_block16(sL, sM, sT, j0, factor);
+      const int bad = potrf_block16<POTRF_LD, POTRF_LD>(sL + j0 * LD + j0, sM + j0 * LD + j0, sT, factor);
       if (lane == 0 && bad >= 0 && j0 + bad < b) atomicCAS(&ra.ctl[2], 0, info_base + j0 + bad + 1);
       POTRF_STAMP(2);
     } else {
       if (below) {
         const int rb = j0 + 16 * warp;  // warps 1, 2: the panel rows below block J
-        if (rb < NB) potrf_panel_rows(sL, sM, jp, rb);
+        if (rb < NB) potrf_panel_rows<LD, LD>(sL + jp * LD, sM + jp * LD + jp, rb);
         named_bar_sync(1, NTHREADS);
         // rows >= j1, columns >= j0, lower part, from the panel of block J-1
         const int nti = (NB - j1) / 16, ntj = (NB - j0) / 8;
         for (int tt = warp - 1; tt < nti * ntj; tt += NTHREADS / 32 - 1) {
           const int r0 = j1 + 16 * (tt / ntj), c0 = j0 + 8 * (tt % ntj);
-          if (c0 <= r0 + 15) potrf_syrk_tile(sL, jp, r0, c0);
+          if (c0 <= r0 + 15) potrf_syrk_tile<LD>(sL, jp, r0, c0);
         }
       }
       if (want_inv && J >= 2)
@@ -1881,44 +1885,120 @@ static __device__ void run_asm(const RunArgs& ra, const Task& t, double* smem) {
 }
 
 // A whole small cholesky front (T_FRONT, nj <= TILE; cholesky.c:33-72 for
-// one node) in shared memory, F(r, c) at F[c*FLD + r], lower part:
-//   1. F = the block's lower trapezoid (columns < nn), zero elsewhere;
+// one node) in shared memory: F(r, c) at F[c * FRONT_LD + r], lower part, the
+// nn pivot columns padded with an identity to NP, a multiple of 16, and the
+// separators from row and column NP on.
+//   1. F = the block's lower trapezoid, zero elsewhere;
 //   2. the children's update matrices added, last child first;
-//   3. the first nn columns eliminated (right-looking: pivot, column scaled,
-//      trailing lower part updated, a warp per column), which leaves L11,
-//      L21 and the Schur complement F22 - L21 L21^T;
+//   3. the pivot columns eliminated in 16-column blocks as in the diagonal
+//      tile tasks (run_potrf), the separators as further rows below them,
+//      which leaves L11, L21 and the Schur complement F22 - L21 L21^T;
 //   4. the rows below replaced by W = L21 L11^{-1} (the reference's layout
-//      of the off-diagonal block), one row per thread;
+//      of the off-diagonal block): by 16-column blocks, last to first,
+//      W_J = (L21_J - sum_{K > J} W_K L(K, J)) Minv_JJ, a warp per 16 rows;
 //   5. the block and the update matrix (operand c) written back.
 // A non-positive pivot records ctl[2] = j + 1 and continues with 1.
-constexpr int FLD = TILE + 1;
-static_assert(2 * TILE * FLD + TILE / 2 <= ENGINE_SMEM_BASE_DOUBLES, "small fronts exceed the engine's shared memory");
+// Bound by its chain of steps: with a barrier a pivot and scalar updates a
+// front of 2-D 30^2 (merged) took 34.2 us, in blocks 13.7.
+constexpr int FRONT_LD = TILE + 20;             // up to 80 rows; 4 mod 16
+constexpr int FRONT_DLD = 20;                   // the inverses of the diagonal blocks
+constexpr int FRONT_D = (TILE + 16) * FRONT_LD;
+static_assert(FRONT_D + TILE * FRONT_DLD + 64 + TILE / 2 <= ENGINE_SMEM_BASE_DOUBLES,
+              "small fronts exceed the engine's shared memory");
+
+// Up to this many pivots are eliminated one by one (a padded block of 16 costs
+// about as much as six of them; 4 and 8 measured the same on 2-D grids, 12
+// 4 % slower).
+constexpr int FRONT_SCALAR_NN = 4;
+
+// Steps 3 and 4 of run_front for a few pivots, column by column with one
+// barrier a pivot: pivot j updates the trailing part with its unscaled
+// column, F(i, c) -= F(i, j) F(c, j) / d_j, and the column itself is scaled by
+// 1 / L(j, j) in the next pivot's phase (nobody reads it then);
+// 1 / L(j, j) = rsqrt(d_j), kept (in w, with L(j, j)) for the solve.
+__device__ __forceinline__ void front_scalar(const RunArgs& ra, double* F, double* w, int nn, int nj) {
+  constexpr int LD = FRONT_LD, NW = NTHREADS / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double* rl = w;
+  double* lj = w + FRONT_SCALAR_NN;
+  int first_bad = -1;
+  for (int j = 0; j < nn; j++) {
+    const double d = F[j * LD + j];
+    const bool bad = !(d > 0.0);
+    if (bad && first_bad < 0) first_bad = j;
+    const double rs = rsqrt(bad ? 1.0 : d), rd = rs * rs;
+    if (j > 0) {
+      const double rp = rl[j - 1];
+      for (int i = j + tid; i < nj; i += NTHREADS) F[(j - 1) * LD + i] *= rp;
+    }
+    if (tid == 0) {
+      rl[j] = rs;  // read from the next phase on
+      lj[j] = (bad ? 1.0 : d) * rs;
+    }
+    for (int c = j + 1 + warp; c < nj; c += NW) {
+      const double fc = F[j * LD + c] * rd;
+      for (int i = c + lane; i < nj; i += 32) F[c * LD + i] -= F[j * LD + i] * fc;
+    }
+    __syncthreads();
+  }
+  for (int i = nn + tid; i < nj; i += NTHREADS) F[(nn - 1) * LD + i] *= rl[nn - 1];
+  for (int j = tid; j < nn; j += NTHREADS) F[j * LD + j] = lj[j];
+  if (tid == 0 && first_bad >= 0) atomicCAS(&ra.ctl[2], 0, first_bad + 1);
+  __syncthreads();
+  // W = L21 L11^{-1}, one row per thread, right-looking: w_j = t_j / L(j, j),
+  // then t_j' -= w_j L(j, j') for j' < j (independent updates)
+  for (int i = nn + tid; i < nj; i += NTHREADS)
+    for (int j = nn - 1; j >= 0; j--) {
+      const double v = F[j * LD + i] * rl[j];
+      F[j * LD + i] = v;
+      for (int l2 = 0; l2 < j; l2++) F[l2 * LD + i] -= v * F[l2 * LD + j];
+    }
+  __syncthreads();
+}
 
 static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem) {
+  constexpr int LD = FRONT_LD, LDM = FRONT_DLD, NW = NTHREADS / 32;
   const FrontDesc f = ra.fronts[t.aux[0]];
   const int nn = f.nn, na = f.na, nj = f.nj;
+  const bool blocked = nn > FRONT_SCALAR_NN;
+  const int NJ = blocked ? (nn + 15) >> 4 : 0, NP = blocked ? 16 * NJ : nn, pad = NP - nn;
+  const int NB = (NP + na + 15) >> 4, NF = blocked ? 16 * NB : nj;  // order of F
   double* F = smem;
+  double* D = smem + FRONT_D;         // block J's inverse at D + J * 16 * LDM
+  double* sT = D + TILE * LDM;
+  int* sr = reinterpret_cast<int*>(sT + 64);
   double* __restrict__ X = ra.bases[t.a.base] + t.a.off;
   double* __restrict__ U = ra.bases[t.c.base] + t.c.off;
   const int ldu = t.c.ld;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NW = NTHREADS / 32;
-  for (int c = warp; c < nj; c += NW)
-    for (int r = lane; r < nj; r += 32)
-      F[c * FLD + r] = (c < nn && r >= c) ? __ldcg(X + (int64_t)c * nj + r) : 0.0;
+  // F by column: a pivot column's trapezoid, an identity column or zeros
+  for (int c = warp; c < NF; c += NW) {
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+      const int r = lane + 32 * e;  // row of F; of the block: r or r - pad
+      if (r >= NF) continue;
+      const int rb = r < NP ? r : r - pad;
+      const bool in = c < nn && r >= c && (r < nn || (r >= NP && rb < nj));
+      F[c * LD + r] = in ? __ldcg(X + (int64_t)c * nj + rb) : (r == c && c >= nn && c < NP ? 1.0 : 0.0);
+    }
+  }
+  if (blocked)
+    for (int i = tid; i < NP * LDM; i += NTHREADS) D[i] = 0.0;
   __syncthreads();
   // the children's update matrices, last child first: its relative indices
   // staged in shared memory, then the lower triangle of U_c flattened over
   // the threads with FRONT_E loads in flight per thread (a child's entries
   // land on distinct front entries)
   constexpr int FRONT_E = 8;
-  int* sr = reinterpret_cast<int*>(F + TILE * FLD + 2 * TILE);
   for (int l = f.chend - 1; l >= f.chbeg; l--) {
     const FrontDesc ch = ra.fronts[ra.chidx[l]];
     const int Nc = ch.na, tot = Nc * Nc;
     const int32_t* __restrict__ rr = ra.relidx + ch.relptr;
     const double* __restrict__ Uc = ra.bases[B_WS] + t.off2 + ch.upd;
-    if (tid < Nc) sr[tid] = __ldg(rr + tid);
+    if (tid < Nc) {
+      const int r = __ldg(rr + tid);
+      sr[tid] = r < nn ? r : r + pad;
+    }
     __syncthreads();
     for (int base = 0; base < tot; base += FRONT_E * NTHREADS) {
       double v[FRONT_E];
@@ -1928,7 +2008,7 @@ static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem)
         const int idx = base + tid + e * NTHREADS, q = idx / Nc, i = idx - q * Nc;
         const bool ok = idx < tot && i >= q;
         v[e] = ok ? __ldcg(Uc + idx) : 0.0;
-        dst[e] = ok ? sr[q] * FLD + sr[i] : -1;
+        dst[e] = ok ? sr[q] * LD + sr[i] : -1;
       }
 #pragma unroll
       for (int e = 0; e < FRONT_E; e++)
@@ -1936,130 +2016,243 @@ static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem)
     }
     __syncthreads();
   }
-  // Pivots with one barrier each: pivot j updates the trailing part with
-  // its unscaled column, F(i, c) -= F(i, j) F(c, j) / d_j, and the column
-  // itself is scaled by 1 / L(j, j) in the next pivot's phase (nobody reads
-  // it then); 1 / L(j, j) = rsqrt(d_j), kept for the solve below.
-  // The diagonal entries L(j, j) = d_j / sqrt(d_j) are written after the
-  // loop (every thread reads d_j in pivot j's phase).
-  double* rl = F + TILE * FLD;  // 1 / L(j, j)
-  double* lj = rl + TILE;       // L(j, j)
-  int first_bad = -1;
-  for (int j = 0; j < nn; j++) {
-    const double d = F[j * FLD + j];
-    const bool bad = !(d > 0.0);
-    if (bad && first_bad < 0) first_bad = j;
-    const double rs = rsqrt(bad ? 1.0 : d), rd = rs * rs;
-    if (j > 0) {
-      const double rp = rl[j - 1];
-      for (int i = j + tid; i < nj; i += NTHREADS) F[(j - 1) * FLD + i] *= rp;
-    }
-    if (tid == 0) {
-      rl[j] = rs;  // read from the next phase on
-      lj[j] = (bad ? 1.0 : d) * rs;
-    }
-    for (int c = j + 1 + warp; c < nj; c += NW) {
-      const double fc = F[j * FLD + c] * rd;
-      for (int i = c + lane; i < nj; i += 32) F[c * FLD + i] -= F[j * FLD + i] * fc;
+  if (!blocked) {
+    front_scalar(ra, F, D, nn, nj);
+  }
+  // step J: warp 0 the panel rows, the update and the factor of diagonal
+  // block J, warps 1-3 the other panel rows of block J - 1 and the updates
+  // below (one more step, of all warps, for the separators' rows and columns)
+#pragma unroll 1
+  for (int J = 0; J < NJ; J++) {
+    const int j0 = 16 * J, jp = j0 - 16;
+    const double* Mp = D + (J - 1) * 16 * LDM;
+    if (warp == 0) {
+      if (J > 0) {
+        potrf_panel_rows<LD, LDM>(F + jp * LD, Mp, j0);
+        named_bar_arrive(1, NTHREADS);
+        potrf_syrk_tile<LD>(F, jp, j0, j0);
+        potrf_syrk_tile<LD>(F, jp, j0, j0 + 8);
+        __syncwarp();
+      }
+      const int bad = potrf_block16<LD, LDM>(F + j0 * LD + j0, D + J * 16 * LDM, sT, true, min(16, nn - j0));
+      if (lane == 0 && bad >= 0) atomicCAS(&ra.ctl[2], 0, j0 + bad + 1);
+    } else if (J > 0) {
+      for (int rb = J + warp; rb < NB; rb += NW - 1) potrf_panel_rows<LD, LDM>(F + jp * LD, Mp, 16 * rb);
+      named_bar_sync(1, NTHREADS);
+      int at = 0;
+      for (int I = J + 1; I < NB; I++)
+        for (int c0 = j0; c0 < 16 * I + 16; c0 += 8)
+          if (at++ % (NW - 1) == warp - 1) potrf_syrk_tile<LD>(F, jp, 16 * I, c0);
     }
     __syncthreads();
   }
-  if (nn > 0)
-    for (int i = nn + tid; i < nj; i += NTHREADS) F[(nn - 1) * FLD + i] *= rl[nn - 1];
-  for (int j = tid; j < nn; j += NTHREADS) F[j * FLD + j] = lj[j];
-  if (tid == 0 && first_bad >= 0) atomicCAS(&ra.ctl[2], 0, first_bad + 1);
-  __syncthreads();
-  // W = L21 L11^{-1}, one row per thread, right-looking: w_j = t_j / L(j, j),
-  // then t_j' -= w_j L(j, j') for j' < j (independent updates)
-  for (int i = nn + tid; i < nj; i += NTHREADS)
-    for (int j = nn - 1; j >= 0; j--) {
-      const double v = F[j * FLD + i] * rl[j];
-      F[j * FLD + i] = v;
-      for (int l2 = 0; l2 < j; l2++) F[l2 * FLD + i] -= v * F[l2 * FLD + j];
+  if (blocked && na > 0) {
+    const int jp = NP - 16;
+    for (int rb = NJ + warp; rb < NB; rb += NW) potrf_panel_rows<LD, LDM>(F + jp * LD, D + (NJ - 1) * 16 * LDM, 16 * rb);
+    __syncthreads();
+    int at = 0;
+    for (int I = NJ; I < NB; I++)
+      for (int c0 = NP; c0 < 16 * I + 16; c0 += 8)
+        if (at++ % NW == warp) potrf_syrk_tile<LD>(F, jp, 16 * I, c0);
+    __syncthreads();
+    const int g = lane >> 2, q = lane & 3;
+    for (int rb = NJ + warp; rb < NB; rb += NW) {
+      const int r0 = 16 * rb;
+#pragma unroll 1
+      for (int J = NJ - 1; J >= 0; J--) {
+        double* const d = F + (16 * J + 2 * q) * LD + r0 + g;
+        double acc[2][4];
+        if (J < NJ - 1) {
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+#pragma unroll
+            for (int h = 0; h < 4; h++) acc[e][h] = d[(8 * e + (h & 1)) * LD + (h & 2) * 4];
+            for (int K = J + 1; K < NJ; K++)
+              warp_mma_16x8<true>(acc[e], F + 16 * K * LD + r0, LD, F + (16 * J + 8 * e) * LD + 16 * K, 1, LD, 16);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int e = 0; e < 2; e++)
+#pragma unroll
+            for (int h = 0; h < 4; h++) d[(8 * e + (h & 1)) * LD + (h & 2) * 4] = acc[e][h];
+          __syncwarp();
+        }
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+#pragma unroll
+          for (int h = 0; h < 4; h++) acc[e][h] = 0.0;
+          warp_mma_16x8<false>(acc[e], F + 16 * J * LD + r0, LD, D + J * 16 * LDM + 8 * e * LDM, 1, LDM, 16);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+#pragma unroll
+          for (int h = 0; h < 4; h++) d[(8 * e + (h & 1)) * LD + (h & 2) * 4] = acc[e][h];
+        __syncwarp();
+      }
     }
-  __syncthreads();
+    __syncthreads();
+  }
   for (int c = warp; c < nn; c += NW)
-    for (int r = c + lane; r < nj; r += 32) X[(int64_t)c * nj + r] = F[c * FLD + r];
+    for (int r = c + lane; r < nj; r += 32) X[(int64_t)c * nj + r] = F[c * LD + (r < nn ? r : r + pad)];
   for (int q = warp; q < na; q += NW)
-    for (int i = q + lane; i < na; i += 32) U[(int64_t)q * ldu + i] = F[(nn + q) * FLD + nn + i];
+    for (int i = q + lane; i < na; i += 32) U[(int64_t)q * ldu + i] = F[(NP + q) * LD + NP + i];
+}
+
+// acc += A(16 x K) B(K x 8) (NEG: -=) over k0 <= k < K with
+// A(r, k) = pa[r * ras + k * kas] and B(k, n) = pb[k * kbs + n * nbs] in shared
+// memory, in two chains of MMAs; k0 a multiple of 8, any K.
+template <bool NEG>
+__device__ __forceinline__ void warp_mma_any(double (&acc)[4], const double* pa, int ras, int kas, const double* pb,
+                                             int kbs, int nbs, int k0, int K) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  double odd[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+  for (int k = k0; k < K; k += 8) {
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int kk = k + 4 * e + q;
+      const bool ok = kk < K;
+      const double a0 = ok ? pa[g * ras + kk * kas] : 0.0, a1 = ok ? pa[(g + 8) * ras + kk * kas] : 0.0;
+      const double b0 = ok ? pb[kk * kbs + g * nbs] : 0.0;
+      dmma16(e ? odd : acc, NEG ? -a0 : a0, NEG ? -a1 : a1, b0);
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 4; h++) acc[h] += odd[h];
 }
 
 // A whole small projected-inverse front (T_PFRONT, nj <= TILE;
-// projected_inverse.c:33-73 for one node) in two shared-memory buffers of
-// leading dimension FLD: G holds L11, then M = L11^{-1} (inverted in place,
-// columns last to first, as LAPACK's unblocked triangular inverse does),
-// then S21; F holds the front: W and V_k (operand c) first, then
-// [Y11; S21 | V_k].
-//   Y11 = M^T M;  S21 = -V_k W;  Y11 -= S21^T W;
+// projected_inverse.c:33-73 for one node) in shared memory: G holds L11,
+// padded with an identity to a multiple of 16 columns, then M = L11^{-1} in
+// its place (diagonal 16 x 16 blocks by a warp each, then block row by block
+// row), then S21; F holds the front: W and V_k (operand c, both triangles)
+// first, then [Y11; S21 | V_k].
+//   Y11 = M^T M;  S21 = -V_k W;  Y11 -= S21^T W   (FP64 MMAs);
 //   U_c = F(r_c, r_c) for every child c (lower parts);
 //   the block <- [Y11 (strict upper part zeroed); S21].
 // A zero diagonal entry records ctl[2] = j + 1 and is taken as 1.
+// With scalar dots, two barriers a column of M, a front of 2-D 30^2 (merged)
+// took 24.1 us, now 12.0.
+constexpr int PF_LD = TILE + 4;
+static_assert(2 * TILE * PF_LD + 4 * 64 + TILE / 2 + 8 <= ENGINE_SMEM_BASE_DOUBLES,
+              "small fronts exceed the engine's shared memory");
 static __device__ void run_pfront(const RunArgs& ra, const Task& t, double* smem) {
+  constexpr int LD = PF_LD, NW = NTHREADS / 32;
   const FrontDesc f = ra.fronts[t.aux[0]];
   const int nn = f.nn, na = f.na, nj = f.nj;
-  double* G = smem;
-  double* F = smem + TILE * FLD;
+  const int NJ = (nn + 15) >> 4, NP = 16 * NJ;
+  double* F = smem;
+  double* G = smem + TILE * LD;
+  double* sT = G + TILE * LD;
+  int* sr = reinterpret_cast<int*>(sT + NW * 64);
+  int* s_bad = sr + TILE;
   double* __restrict__ X = ra.bases[t.a.base] + t.a.off;
   const double* __restrict__ V = ra.bases[t.c.base] + t.c.off;
   const int ldv = t.c.ld;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NW = NTHREADS / 32;
-  for (int c = warp; c < nn; c += NW)
-    for (int r = lane; r < nj; r += 32) {
-      const double v = __ldcg(X + (int64_t)c * nj + r);
-      if (r < nn) G[c * FLD + r] = (r >= c) ? v : 0.0;
-      else F[c * FLD + r] = v;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  if (tid == 0) *s_bad = -1;
+  for (int c = warp; c < NP; c += NW)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int r = lane + 32 * e;
+      const double v = (c < nn && r < nj) ? __ldcg(X + (int64_t)c * nj + r) : 0.0;
+      if (r < NP) G[c * LD + r] = (c < nn && r < nn) ? (r >= c ? v : 0.0) : (r == c ? 1.0 : 0.0);
+      if (c < nn && r >= nn && r < nj) F[c * LD + r] = v;
     }
-  for (int q = warp; q < na; q += NW)
-    for (int i = q + lane; i < na; i += 32) F[(nn + q) * FLD + nn + i] = __ldcg(V + (int64_t)q * ldv + i);
+  for (int c = warp; c < na; c += NW)
+    for (int i = c + lane; i < na; i += 32) {
+      const double v = __ldcg(V + (int64_t)c * ldv + i);
+      F[(nn + c) * LD + nn + i] = v;
+      F[(nn + i) * LD + nn + c] = v;
+    }
   __syncthreads();
-  int first_bad = -1;
-  for (int j = nn - 1; j >= 0; j--) {
-    const double d = G[j * FLD + j];
-    if (d == 0.0 && first_bad < 0) first_bad = j;
-    const double ajj = 1.0 / (d == 0.0 ? 1.0 : d);
-    const int i = j + 1 + tid;
-    double ti = 0.0;
-    if (i < nn)
-      for (int l = j + 1; l <= i; l++) ti = fma(G[l * FLD + i], G[j * FLD + l], ti);
+  if (tid < nn && G[tid * LD + tid] == 0.0) atomicMax(s_bad, tid);
+  __syncthreads();
+  if (tid == 0 && *s_bad >= 0) atomicCAS(&ra.ctl[2], 0, *s_bad + 1);
+  // M in place of L11
+  if (warp < NJ) {
+    double* d = G + 16 * warp * LD + 16 * warp;
+    potrf_block16<LD, LD>(d, d, sT + 64 * warp, false, min(16, nn - 16 * warp));
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int I = 1; I < NJ; I++) {
+    // L(I, :I) M(:I, tile) of at most two tiles a warp, then in their place
+    double ac[2][4];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int tj = warp + NW * e;
+      ac[e][0] = ac[e][1] = ac[e][2] = ac[e][3] = 0.0;
+      if (tj < 2 * I) warp_mma_any<false>(ac[e], G + 16 * I, 1, LD, G + 8 * tj * LD, 1, LD, 16 * (tj / 2), 16 * I);
+    }
     __syncthreads();
-    if (i < nn) G[j * FLD + i] = -ajj * ti;
-    if (tid == 0) G[j * FLD + j] = ajj;
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int tj = warp + NW * e;
+      if (tj >= 2 * I) continue;
+      double* d = G + (8 * tj + 2 * q) * LD + 16 * I + g;
+#pragma unroll
+      for (int h = 0; h < 4; h++) d[(h & 1) * LD + (h & 2) * 4] = ac[e][h];
+      __syncwarp();
+      potrf_inv_finish(G, I, tj);
+    }
     __syncthreads();
   }
-  if (tid == 0 && first_bad >= 0) atomicCAS(&ra.ctl[2], 0, first_bad + 1);
-  for (int j = warp; j < nn; j += NW)
-    for (int i = j + lane; i < nn; i += 32) {
-      double v = 0.0;
-      for (int l = i; l < nn; l++) v = fma(G[i * FLD + l], G[j * FLD + l], v);
-      F[j * FLD + i] = v;
+  // Y11 = M^T M: tiles of 16 x 8 on and below the diagonal
+  int at = 0;
+  for (int I = 0; I < NJ; I++)
+    for (int c0 = 0; c0 < min(16 * I + 16, nn); c0 += 8) {
+      if (at++ % NW != warp) continue;
+      double y[4] = {0.0, 0.0, 0.0, 0.0};
+      warp_mma_any<false>(y, G + 16 * I * LD, LD, 1, G + c0 * LD, 1, LD, 16 * I, NP);
+#pragma unroll
+      for (int h = 0; h < 4; h++) {
+        const int r = 16 * I + g + (h & 2) * 4, c = c0 + 2 * q + (h & 1);
+        if (r < nn && c <= r) F[c * LD + r] = y[h];
+      }
     }
   __syncthreads();
   if (na > 0) {
-    for (int j = warp; j < nn; j += NW)
-      for (int i = lane; i < na; i += 32) {
-        double v = 0.0;
-        for (int l = 0; l < na; l++) {
-          const double vil = (i >= l) ? F[(nn + l) * FLD + nn + i] : F[(nn + i) * FLD + nn + l];
-          v = fma(vil, F[j * FLD + nn + l], v);
+    // S21 = -V W into G
+    at = 0;
+    for (int r0 = 0; r0 < na; r0 += 16)
+      for (int c0 = 0; c0 < nn; c0 += 8) {
+        if (at++ % NW != warp) continue;
+        double y[4] = {0.0, 0.0, 0.0, 0.0};
+        warp_mma_any<true>(y, F + nn * LD + nn + r0, 1, LD, F + c0 * LD + nn, 1, LD, 0, na);
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+          const int r = r0 + g + (h & 2) * 4, c = c0 + 2 * q + (h & 1);
+          if (r < na && c < nn) G[c * LD + r] = y[h];
         }
-        G[j * FLD + i] = -v;
+      }
+    __syncthreads();
+    // Y11 -= S21^T W
+    at = 0;
+    for (int I = 0; I < NJ; I++)
+      for (int c0 = 0; c0 < min(16 * I + 16, nn); c0 += 8) {
+        if (at++ % NW != warp) continue;
+        double y[4];
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+          const int r = 16 * I + g + (h & 2) * 4, c = c0 + 2 * q + (h & 1);
+          y[h] = (r < nn && c <= r) ? F[c * LD + r] : 0.0;
+        }
+        warp_mma_any<true>(y, G + 16 * I * LD, LD, 1, F + c0 * LD + nn, 1, LD, 0, na);
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+          const int r = 16 * I + g + (h & 2) * 4, c = c0 + 2 * q + (h & 1);
+          if (r < nn && c <= r) F[c * LD + r] = y[h];
+        }
       }
     __syncthreads();
     for (int j = warp; j < nn; j += NW)
-      for (int i = j + lane; i < nn; i += 32) {
-        double v = 0.0;
-        for (int l = 0; l < na; l++) v = fma(G[i * FLD + l], F[j * FLD + nn + l], v);
-        F[j * FLD + i] -= v;
-      }
-    __syncthreads();
-    for (int j = warp; j < nn; j += NW)
-      for (int i = lane; i < na; i += 32) F[j * FLD + nn + i] = G[j * FLD + i];
+      for (int i = lane; i < na; i += 32) F[j * LD + nn + i] = G[j * LD + i];
     __syncthreads();
   }
   // the children's updates V_c = F(r_c, r_c), lower triangle, the relative
   // indices staged in shared memory per child
-  int* sr = reinterpret_cast<int*>(smem + 2 * TILE * FLD);
   for (int l = f.chbeg; l < f.chend; l++) {
     const FrontDesc ch = ra.fronts[ra.chidx[l]];
     const int Nc = ch.na, tot = Nc * Nc;
@@ -2068,14 +2261,14 @@ static __device__ void run_pfront(const RunArgs& ra, const Task& t, double* smem
     if (tid < Nc) sr[tid] = __ldg(rr + tid);
     __syncthreads();
     for (int idx = tid; idx < tot; idx += NTHREADS) {
-      const int q = idx / Nc, i = idx - q * Nc;
-      if (i >= q) Uc[idx] = F[sr[q] * FLD + sr[i]];
+      const int c = idx / Nc, i = idx - c * Nc;
+      if (i >= c) Uc[idx] = F[sr[c] * LD + sr[i]];
     }
     __syncthreads();
   }
   for (int c = warp; c < nn; c += NW)
     for (int r = lane; r < nj; r += 32)
-      X[(int64_t)c * nj + r] = (r < nn && r < c) ? 0.0 : F[c * FLD + r];
+      X[(int64_t)c * nj + r] = (r < nn && r < c) ? 0.0 : F[c * LD + r];
 }
 
 // Gather of a child's update matrix out of its parent's front
