@@ -1972,15 +1972,26 @@ static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem)
   const int ldu = t.c.ld;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // F by column: a pivot column's trapezoid, an identity column or zeros
-  for (int c = warp; c < NF; c += NW) {
+  // (four columns' loads at a time: a load is not moved above a store to
+  // shared memory)
+  for (int c4 = warp; c4 < NF; c4 += 4 * NW) {
+    double v[4][3];
 #pragma unroll
-    for (int e = 0; e < 3; e++) {
-      const int r = lane + 32 * e;  // row of F; of the block: r or r - pad
-      if (r >= NF) continue;
-      const int rb = r < NP ? r : r - pad;
-      const bool in = c < nn && r >= c && (r < nn || (r >= NP && rb < nj));
-      F[c * LD + r] = in ? __ldcg(X + (int64_t)c * nj + rb) : (r == c && c >= nn && c < NP ? 1.0 : 0.0);
-    }
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int e = 0; e < 3; e++) {
+        const int c = c4 + u * NW, r = lane + 32 * e;  // row of F; of the block: r or r - pad
+        const int rb = r < NP ? r : r - pad;
+        const bool in = c < nn && r >= c && (r < nn || (r >= NP && rb < nj));
+        v[u][e] = in ? __ldcg(X + (int64_t)c * nj + rb) : (r == c && c >= nn && c < NP ? 1.0 : 0.0);
+      }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int e = 0; e < 3; e++) {
+        const int c = c4 + u * NW, r = lane + 32 * e;
+        if (c < NF && r < NF) F[c * LD + r] = v[u][e];
+      }
   }
   if (blocked)
     for (int i = tid; i < NP * LDM; i += NTHREADS) D[i] = 0.0;
@@ -2152,20 +2163,46 @@ static __device__ void run_pfront(const RunArgs& ra, const Task& t, double* smem
   const int ldv = t.c.ld;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   if (tid == 0) *s_bad = -1;
-  for (int c = warp; c < NP; c += NW)
+  // (four columns' loads at a time: a load is not moved above a store to
+  // shared memory)
+  for (int c4 = warp; c4 < NP; c4 += 4 * NW) {
+    double v[4][2];
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const int r = lane + 32 * e;
-      const double v = (c < nn && r < nj) ? __ldcg(X + (int64_t)c * nj + r) : 0.0;
-      if (r < NP) G[c * LD + r] = (c < nn && r < nn) ? (r >= c ? v : 0.0) : (r == c ? 1.0 : 0.0);
-      if (c < nn && r >= nn && r < nj) F[c * LD + r] = v;
-    }
-  for (int c = warp; c < na; c += NW)
-    for (int i = c + lane; i < na; i += 32) {
-      const double v = __ldcg(V + (int64_t)c * ldv + i);
-      F[(nn + c) * LD + nn + i] = v;
-      F[(nn + i) * LD + nn + c] = v;
-    }
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = c4 + u * NW, r = lane + 32 * e;
+        v[u][e] = (c < nn && r < nj) ? __ldcg(X + (int64_t)c * nj + r) : 0.0;
+      }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = c4 + u * NW, r = lane + 32 * e;
+        if (r < NP) G[c * LD + r] = (c < nn && r < nn) ? (r >= c ? v[u][e] : 0.0) : (r == c ? 1.0 : 0.0);
+        if (c < nn && r >= nn && r < nj) F[c * LD + r] = v[u][e];
+      }
+  }
+  for (int c4 = warp; c4 < na; c4 += 4 * NW) {
+    double v[4][2];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = c4 + u * NW, i = lane + 32 * e;
+        v[u][e] = (c < na && i >= c && i < na) ? __ldcg(V + (int64_t)c * ldv + i) : 0.0;
+      }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = c4 + u * NW, i = lane + 32 * e;
+        if (c < na && i >= c && i < na) {
+          F[(nn + c) * LD + nn + i] = v[u][e];
+          F[(nn + i) * LD + nn + c] = v[u][e];
+        }
+      }
+  }
   __syncthreads();
   if (tid < nn && G[tid * LD + tid] == 0.0) atomicMax(s_bad, tid);
   __syncthreads();
@@ -3003,6 +3040,29 @@ __device__ __forceinline__ int bundle_last(const Task& t, int w) {
   return w == 0 ? t.m : w == 1 ? t.n : w == 2 ? t.k : t.cdiag;
 }
 
+// Global loads go SUB_E at a time into registers before they are stored (a
+// load is not moved above a store to shared memory, so one by one each costs
+// a round trip: a bundle of the 256 uneven grids took 72 us in cholesky and
+// 67 in projected_inverse, now 55 and 63).
+constexpr int SUB_E = 8;
+
+// Columns [c0, c1) of a matrix whose column c begins at src + c * ld, rows
+// >= c, into the lane's row of a front (from entry to0 on); all lanes call.
+__device__ __forceinline__ void sub_load(double* row, const double* __restrict__ src, int ld, int c1, bool lower,
+                                         bool active, int lane, int to0) {
+  for (int c0 = 0; c0 < c1; c0 += SUB_E) {
+    double v[SUB_E];
+#pragma unroll
+    for (int e = 0; e < SUB_E; e++) {
+      const int c = c0 + e;
+      v[e] = (active && c < c1 && (!lower || lane >= c)) ? __ldcg(src + (int64_t)c * ld + lane) : 0.0;
+    }
+#pragma unroll
+    for (int e = 0; e < SUB_E; e++)
+      if (active && c0 + e < c1) row[to0 + c0 + e] = v[e];
+  }
+}
+
 // cholesky.c:33-72 for one front of at most SUB_NJ rows, by one warp.
 static __device__ void chol_front_warp(const RunArgs& ra, int k, double* F, int lane) {
   const FrontDesc f = ra.fronts[k];
@@ -3010,37 +3070,62 @@ static __device__ void chol_front_warp(const RunArgs& ra, int k, double* F, int 
   double* __restrict__ X = ra.bases[B_X] + f.blk;
   double* __restrict__ W = ra.bases[B_WS];
   double* row = F + lane * SUB_LD;
+  sub_load(row, X, nj, nn, true, lane < nj, lane, 0);
   if (lane < nj)
-    for (int c = 0; c < nj; c++) row[c] = (c < nn && lane >= c) ? __ldcg(X + (int64_t)c * nj + lane) : 0.0;
+    for (int c = nn; c < nj; c++) row[c] = 0.0;
   __syncwarp();
   // extend-add, children last to first (the reference's stack order)
   for (int l = f.chend - 1; l >= f.chbeg; l--) {
     const FrontDesc ch = ra.fronts[ra.chidx[l]];
     const int Nc = ch.na;
-    const int32_t* __restrict__ rr = ra.relidx + ch.relptr;
     const double* __restrict__ Uc = W + ch.upd;
-    if (lane < Nc) {
-      double* dst = F + __ldg(rr + lane) * SUB_LD;
-      for (int q = 0; q <= lane; q++) dst[__ldg(rr + q)] += __ldcg(Uc + (int64_t)q * Nc + lane);
+    const int r = lane < Nc ? __ldg(ra.relidx + ch.relptr + lane) : 0;
+    double* dst = F + r * SUB_LD;
+    for (int q0 = 0; q0 < Nc; q0 += SUB_E) {
+      double v[SUB_E];
+      int rq[SUB_E];
+#pragma unroll
+      for (int e = 0; e < SUB_E; e++) {
+        const int q = q0 + e;
+        rq[e] = __shfl_sync(0xffffffffu, r, q & 31);
+        v[e] = (lane < Nc && q <= lane) ? __ldcg(Uc + (int64_t)q * Nc + lane) : 0.0;
+      }
+#pragma unroll
+      for (int e = 0; e < SUB_E; e++)
+        if (lane < Nc && q0 + e <= lane) dst[rq[e]] += v[e];
     }
     __syncwarp();
   }
   // partial Cholesky of the nn pivot columns; the trailing block becomes U_k
+  // (1 / L(j, j) is kept behind row j)
   int first_bad = -1;
   for (int j = 0; j < nn; j++) {
     const double d = F[j * SUB_LD + j];
     const bool bad = !(d > 0.0);
     if (bad && first_bad < 0) first_bad = j;
-    const double lj = sqrt(bad ? 1.0 : d), rl = 1.0 / lj;
+    const double x = bad ? 1.0 : d, rs = rsqrt(x);
     double a = 0.0;
     if (lane > j && lane < nj) {
-      a = row[j] * rl;
+      a = row[j] * rs;
       row[j] = a;
     }
     __syncwarp();
-    if (lane == j) row[j] = lj;
-    if (lane > j && lane < nj)
-      for (int c = j + 1; c <= lane; c++) row[c] -= a * F[c * SUB_LD + j];
+    if (lane == j) {
+      row[j] = x * rs;
+      row[SUB_NJ] = rs;
+    }
+    for (int c0 = j + 1; c0 < nj; c0 += SUB_E) {
+      double u[SUB_E], w[SUB_E];
+#pragma unroll
+      for (int e = 0; e < SUB_E; e++) {
+        const int c = min(c0 + e, nj - 1);
+        u[e] = F[c * SUB_LD + j];
+        w[e] = row[c];
+      }
+#pragma unroll
+      for (int e = 0; e < SUB_E; e++)
+        if (c0 + e <= lane && lane < nj) row[c0 + e] = fma(-a, u[e], w[e]);
+    }
     __syncwarp();
   }
   if (lane == 0 && first_bad >= 0) atomicCAS(&ra.ctl[2], 0, first_bad + 1);
@@ -3048,8 +3133,8 @@ static __device__ void chol_front_warp(const RunArgs& ra, int k, double* F, int 
   if (lane >= nn && lane < nj)
     for (int j = nn - 1; j >= 0; j--) {
       double v = row[j];
-      for (int l2 = j + 1; l2 < nn; l2++) v -= row[l2] * F[l2 * SUB_LD + j];
-      row[j] = v / F[j * SUB_LD + j];
+      for (int l2 = j + 1; l2 < nn; l2++) v = fma(-row[l2], F[l2 * SUB_LD + j], v);
+      row[j] = v * F[j * SUB_LD + SUB_NJ];
     }
   __syncwarp();
   for (int c = 0; c < nn; c++)
@@ -3069,14 +3154,9 @@ static __device__ void pinv_front_warp(const RunArgs& ra, int k, double* G, doub
   double* __restrict__ X = ra.bases[B_X] + f.blk;
   double* __restrict__ W = ra.bases[B_WS];
   const double* __restrict__ V = W + f.upd;
-  if (lane < nj)
-    for (int c = 0; c < nn; c++) {
-      const double v = __ldcg(X + (int64_t)c * nj + lane);
-      if (lane < nn) G[lane * SUB_LD + c] = (lane >= c) ? v : 0.0;
-      else F[lane * SUB_LD + c] = v;
-    }
-  if (lane < na)
-    for (int q = 0; q <= lane; q++) F[(nn + lane) * SUB_LD + nn + q] = __ldcg(V + (int64_t)q * na + lane);
+  // L11 into G, with zeros above its diagonal; W and V_k into F
+  sub_load((lane < nn ? G : F) + lane * SUB_LD, X, nj, nn, true, lane < nj, lane, 0);
+  sub_load(F + (nn + lane) * SUB_LD, V, na, na, true, lane < na, lane, nn);
   __syncwarp();
   // M = L11^{-1} in place, columns last to first
   int first_bad = -1;
@@ -3129,11 +3209,12 @@ static __device__ void pinv_front_warp(const RunArgs& ra, int k, double* G, doub
   for (int l = f.chbeg; l < f.chend; l++) {
     const FrontDesc ch = ra.fronts[ra.chidx[l]];
     const int Nc = ch.na;
-    const int32_t* __restrict__ rr = ra.relidx + ch.relptr;
     double* __restrict__ Uc = W + ch.upd;
-    if (lane < Nc) {
-      const double* src = F + __ldg(rr + lane) * SUB_LD;
-      for (int q = 0; q <= lane; q++) Uc[(int64_t)q * Nc + lane] = src[__ldg(rr + q)];
+    const int r = lane < Nc ? __ldg(ra.relidx + ch.relptr + lane) : 0;
+    const double* src = F + r * SUB_LD;
+    for (int q = 0; q < Nc; q++) {
+      const int rq = __shfl_sync(0xffffffffu, r, q);
+      if (lane < Nc && q <= lane) Uc[(int64_t)q * Nc + lane] = src[rq];
     }
   }
   for (int c = 0; c < nn; c++)
