@@ -1529,7 +1529,8 @@ __device__ __forceinline__ void mma_rows_lower_b(const double* sA, const double*
   constexpr int LD = POTRF_LD;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
   const int r0 = 16 * warp + g;
-#pragma unroll 1
+  // (unrolled: with j >= kb a branch, every MMA waited for its own load)
+#pragma unroll
   for (int kb = 0; kb < TILE / 8; kb++) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -1665,12 +1666,7 @@ __device__ __forceinline__ void potrf_lookahead(const RunArgs& ra, const Task& t
     }
   }
   POTRF_STAMP(20);
-  // D -= L' L'^T on and below the diagonal
-  double acc[5][4];
-#pragma unroll
-  for (int i = 0; i < 5; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0;
-  mma_lower_tiles(sL, b, acc);
-  POTRF_STAMP(21);
+  // D -= L' L'^T on and below the diagonal; D is loaded beside the product
   double old[5][4];
 #pragma unroll
   for (int i = 0; i < 5; i++) {
@@ -1682,6 +1678,11 @@ __device__ __forceinline__ void potrf_lookahead(const RunArgs& ra, const Task& t
       old[i][h] = (r < m2 && r >= c) ? __ldcg(D + (int64_t)c * lda + r) : 0.0;
     }
   }
+  double acc[5][4];
+#pragma unroll
+  for (int i = 0; i < 5; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0;
+  mma_lower_tiles(sL, b, acc);
+  POTRF_STAMP(21);
 #pragma unroll
   for (int i = 0; i < 5; i++) {
     int rb, j;
