@@ -242,13 +242,18 @@ extern "C" int chb_info(chb_plan* plan, void* work, void* stream) {
   clear_error();
   int rc = check_plan(plan);
   if (rc) return rc;
+  // one wait for the sweep and its status (a wait, then a copy on the default
+  // stream: a sweep of 0.2 ms took 2 us longer, a solve of 0.8 ms 3 us)
+  int ctl[4];
+  const cudaError_t ce = cudaMemcpyAsync(ctl, work, sizeof(ctl), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
   if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) {
     cudaError_t e = cudaGetLastError();
     return set_error(-100 - (int)e, "stream synchronisation failed: %s", cudaGetErrorString(e));
   }
-  int ctl[4];
-  if (cudaMemcpy(ctl, work, sizeof(ctl), cudaMemcpyDeviceToHost) != cudaSuccess)
+  if (ce != cudaSuccess) {
+    cudaGetLastError();
     return set_error(-3, "cannot read the sweep status");
+  }
   if (ctl[1] == DE_TIMEOUT) return set_error(-30, "a task wait timed out (%d CTAs)", ctl[3]);
   if (ctl[1] != 0) return set_error(-31, "device error %d", ctl[1]);
   return ctl[2];
