@@ -52,6 +52,16 @@ int build_trsm(const chb_plan& P, Program& prog, int64_t nrhs, bool trans, bool 
   const int nrt = ceil_div(nrhs, T);  // right-hand-side column tiles
   auto rw = [&](int s) { return (int)std::min<int64_t>(T, nrhs - (int64_t)s * T); };
   const int KC = 128;                 // K chunk of the split long products
+  static_assert(128 <= TRSV_KMAX, "a narrow product is staged whole");
+  // Products of the factor with few right-hand sides are narrow: their part
+  // of the factor is staged in one go, before they wait.  Against 64 x 64
+  // tiles, whose ring takes a round trip per three chunks and fills unused
+  // columns with zeros, a pair of 40^3 solves took 1.45 ms instead of 1.66
+  // with 16 right-hand sides and 2.22 instead of 2.26 with 32, but 3.84
+  // instead of 3.65 with 64, where the tiles' MMAs reuse their operands.
+  auto narrow = [&](Task& t) {
+    if (t.n <= 32 && t.k <= TRSV_KMAX) t.aux[0] = GEMM_NARROW;
+  };
 
   // workspace: Bp (n x nrhs, ld n); u_k (na x nrhs, ld na) per front; per
   // diagonal block c of every front the step operand ('N': [-G2_c | -G_c |
@@ -94,7 +104,9 @@ int build_trsm(const chb_plan& P, Program& prog, int64_t nrhs, bool trans, bool 
   auto split_gemm = [&](const Task& t, const SchedKey& key, int group, std::vector<int>& parts) -> int {
     const int p = split_count(t.k, KC);
     if (p == 1) {
-      const int id = B.add(t, key, group);
+      Task u = t;
+      narrow(u);
+      const int id = B.add(u, key, group);
       parts.push_back(id);
       return id;
     }
@@ -112,6 +124,7 @@ int build_trsm(const chb_plan& P, Program& prog, int64_t nrhs, bool trans, bool 
       u.beta = 0.0;
       u.cmode = CM_FULL;
       u.c = opnd(B_WS, scr + (int64_t)q * T * t.n, T);
+      narrow(u);
       SchedKey kk = key;
       kk.rank = key.rank * 64 + q;
       mine.push_back(B.add(u, kk));
@@ -253,6 +266,7 @@ int build_trsm(const chb_plan& P, Program& prog, int64_t nrhs, bool trans, bool 
     auto far_update = [&](const Operand& a, int r, int c, int s, const SchedKey& key, int sol) {
       Task u = gemm(bw(r), rw(s), bw(c), -1.0, a, xop(c, s, OM_T), 1.0, xop(r, s, OM_N));
       if (!ordered) u.cmode = CM_ATOMIC;
+      narrow(u);
       const int uid = B.add(u, key, far[r * nrt + s]);
       nfar[r * nrt + s]++;
       B.wait_task(uid, sol);
@@ -369,6 +383,7 @@ int build_trsm(const chb_plan& P, Program& prog, int64_t nrhs, bool trans, bool 
             Operand c = opnd(B_WS, uk + i * T + (int64_t)s * T * na, na);
             Task u = gemm(bh(i), rw(s), kq, -1.0, a, shift_k(xop(0, s, OM_T), k0), 1.0, c);
             u.cmode = CM_ATOMIC;
+            narrow(u);
             const int id = B.add(u, {lv, 1, 0, (int)k, s, i}, ugrp[k]);
             wait_x(id);
             B.wait_task(id, zero);
@@ -452,6 +467,7 @@ int build_trsm(const chb_plan& P, Program& prog, int64_t nrhs, bool trans, bool 
               Operand b = opnd(B_WS, uk + (int64_t)s * T * na + k0, na, OM_T);
               Task t = gemm(bw(c), rw(s), kq, -1.0, a, b, 1.0, xop(c, s, OM_N));
               t.cmode = CM_ATOMIC;
+              narrow(t);
               const int id = B.add(t, {lv, 2 * NBc + 2, 0, (int)k, s, c}, xdone);
               B.wait_task(id, prev[s]);
               B.wait_group(id, from_parent);

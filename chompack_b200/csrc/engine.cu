@@ -1,5 +1,5 @@
 // Launch of the persistent kernel, and its build for the FP64 sweeps without
-// Householder panels.
+// Householder panels and solve tasks.
 #include "engine_kernel.cuh"
 
 namespace chb {
@@ -19,12 +19,14 @@ extern "C" int chb_dev_potrf_phase(unsigned long long* out, int clear) {
 }
 #endif
 
-// The other builds (engine_tc.cu, engine_ql.cu).
+// The other builds (engine_tc.cu, engine_ql.cu, engine_solve.cu).
 extern template cudaError_t build_launch<EB_TCGEN05>(const RunArgs&, int, size_t, cudaStream_t);
 extern template cudaError_t build_set_smem<EB_TCGEN05>(size_t);
 extern template cudaError_t build_occupancy<EB_TCGEN05>(int*, size_t);
 extern template cudaError_t build_launch<EB_PANELS>(const RunArgs&, int, size_t, cudaStream_t);
 extern template cudaError_t build_set_smem<EB_PANELS>(size_t);
+extern template cudaError_t build_launch<EB_SOLVE>(const RunArgs&, int, size_t, cudaStream_t);
+extern template cudaError_t build_set_smem<EB_SOLVE>(size_t);
 
 size_t engine_smem_bytes() { return (size_t)ENGINE_SMEM_DOUBLES * sizeof(double); }
 
@@ -34,10 +36,12 @@ size_t engine_smem_bytes() { return (size_t)ENGINE_SMEM_DOUBLES * sizeof(double)
 cudaError_t engine_launch(const RunArgs& ra, int grid, cudaStream_t stream) {
   if (ra.smem_doubles < ENGINE_SMEM_BASE_DOUBLES || ra.smem_doubles > ENGINE_SMEM_DOUBLES) return cudaErrorInvalidValue;
   // the tcgen05 build is sized (engine_occupancy) for the base staging only
-  if (ra.tmem && (ra.panels || ra.smem_doubles != ENGINE_SMEM_BASE_DOUBLES)) return cudaErrorInvalidValue;
+  if (ra.panels && ra.solve) return cudaErrorInvalidValue;
+  if (ra.tmem && (ra.panels || ra.solve || ra.smem_doubles != ENGINE_SMEM_BASE_DOUBLES)) return cudaErrorInvalidValue;
   const size_t smem = (size_t)ra.smem_doubles * sizeof(double);
   if (ra.tmem) return build_launch<EB_TCGEN05>(ra, grid, smem, stream);
   if (ra.panels) return build_launch<EB_PANELS>(ra, grid, smem, stream);
+  if (ra.solve) return build_launch<EB_SOLVE>(ra, grid, smem, stream);
   return build_launch<EB_BASE>(ra, grid, smem, stream);
 }
 
@@ -53,6 +57,7 @@ int engine_occupancy(int* blocks_per_sm, bool tc) {
   cudaError_t e = build_set_smem<EB_BASE>(smem);
   if (e == cudaSuccess) e = build_set_smem<EB_TCGEN05>(smem);
   if (e == cudaSuccess) e = build_set_smem<EB_PANELS>(smem);
+  if (e == cudaSuccess) e = build_set_smem<EB_SOLVE>(smem);
   if (e == cudaSuccess)
     e = tc ? build_occupancy<EB_TCGEN05>(blocks_per_sm, smem_tc) : build_occupancy<EB_BASE>(blocks_per_sm, smem);
   return e == cudaSuccess ? 0 : -1;

@@ -37,11 +37,13 @@ constexpr int MAX_BASES = 64;     // base-pointer slots (see Base below)
 // carve-out, which leaves more L1 for the register spills.
 constexpr int ENGINE_SMEM_BASE_DOUBLES = 9472;
 constexpr int ENGINE_SMEM_DOUBLES = 14336;
-// T_TRSV: the largest K, and the leading dimension of its staged operand;
-// programs with such steps launch with ENGINE_SMEM_DOUBLES
+// T_TRSV: the largest K, and the leading dimensions of its staged operands
+// (4 mod 16 for B, whose MMA fragments then meet no bank twice); programs
+// with such steps launch with ENGINE_SMEM_DOUBLES
 constexpr int TRSV_KMAX = 192;
 constexpr int TRSV_LA = TILE + 2;
-static_assert(TRSV_KMAX * TRSV_LA + TRSV_KMAX * 8 <= ENGINE_SMEM_DOUBLES, "T_TRSV staging exceeds shared memory");
+constexpr int TRSV_LB = TRSV_KMAX + 4;
+static_assert(TRSV_KMAX * TRSV_LA + 8 * TRSV_LB <= ENGINE_SMEM_DOUBLES, "T_TRSV staging exceeds shared memory");
 // Householder panels of h rows.  Up to QL_REG_ROWS rows a panel is reduced in
 // registers, at most 64 entries a thread, which bounds its columns.
 constexpr int QL_REG_ROWS = 512;
@@ -90,6 +92,10 @@ enum CMode : uint8_t {
                  // tasks update at once, in any order
 };
 
+// aux[0] of a T_GEMM whose operand a no task of its program writes, opB is
+// OM_T, n <= 32 and k <= TRSV_KMAX: run as a T_TRSV
+constexpr int GEMM_NARROW = 1;
+
 enum TaskOp : uint8_t {
   T_GEMM = 0,     // C = alpha * opA * opB^T + beta * C
   T_POTRF = 1,    // Cholesky of a diagonal tile; optionally its inverse
@@ -116,9 +122,10 @@ enum TaskOp : uint8_t {
 
 // Builds of the persistent kernel.
 enum EngineBuild : int {
-  EB_BASE = 0,     // FP64 and warp-level TF32 sweeps without Householder panels
+  EB_BASE = 0,     // FP64 and warp-level TF32 sweeps without what follows
   EB_TCGEN05 = 1,  // TF32 tiles on tcgen05
-  EB_PANELS = 2    // programs with T_QL tasks
+  EB_PANELS = 2,   // programs with T_QL tasks
+  EB_SOLVE = 3     // programs with T_VEC and T_TRSV tasks and narrow products
 };
 
 // Sub-operations of T_QL (child aux[0], columns [aux[1], aux[2]) of the
@@ -208,6 +215,7 @@ struct RunArgs {
   int nwords;                     // ready-bitmap words (64 tasks each)
   int nsumm;                      // summary words (64 bitmap words each)
   int panels;                     // 1: the program has Householder panels (T_QL)
+  int solve;                      // 1: the program has solve tasks (T_VEC, T_TRSV)
   int tmem;                       // 1: TF32 GEMM tiles run on tcgen05 (tensor memory allocated per CTA)
   int* pend;                      // unmet dependencies per task
   unsigned long long* ready;      // ready, unclaimed tasks

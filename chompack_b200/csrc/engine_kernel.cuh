@@ -1023,48 +1023,59 @@ static __device__ void run_sum(const RunArgs& ra, const Task& t) {
   }
 }
 
-// C = alpha * M2 * (opA * opB^T), M2 = lower-triangular m x m tile (operand
-// `c` of the task holds C; M2 is described by aux: base aux[0], ld aux[1],
-// offset (aux[2] | aux[3] << 32)).
 // One step of a block substitution (the triangular solves):
 // C (m x n) = alpha A (m x K) B (K x n) + beta C, m <= 64, K <= TRSV_KMAX,
 // with A a step operand computed before the sweep's chain ([-G_c | M_c] or
-// [M_c; -H_c] stored transposed) and B adjacent x tiles, C one of them.
-// A's copies into shared memory (sA[k*TRSV_LA + r], zero outside m x K) are
+// [M_c; -H_c] stored transposed) and B adjacent x tiles, C one of them; or a
+// narrow product of the solves (T_GEMM with aux[0] = GEMM_NARROW, n <= 32,
+// A in the factor, C possibly added into with atomics).
+// A's copies into shared memory (sA[k*TRSV_LA + r], k in [K, K4) zero) are
 // issued before the task's mid waits [cdiag, nwait) (the x tiles it reads,
-// written by the chain), so that they overlap the wait; then B is read in
-// groups of 8 right-hand sides (sB[k*8 + j]) and each warp multiplies its
-// 16 rows with FP64 MMAs.  A wait that runs out sets the timeout status
-// and returns once the copies have landed.
-static __device__ void run_trsv(const RunArgs& ra, const Task& t, double* smem) {
+// written by the chain; all waits of a narrow product under the static
+// order, since the factor is there from the start), so that they overlap the
+// wait.  Then B is read, 8 right-hand sides at a time, a group's up to 12
+// loads a thread in flight together (sB[j*TRSV_LB + k]), and each warp
+// multiplies its 16 rows with FP64 MMAs in four chains.  A wait that runs
+// out sets the timeout status and returns once the copies have landed.
+// Bound by the hops of the chain: a step is an L2 round trip for B, the
+// product and the release.  With B in three dependent groups of loads, one
+// chain of MMAs and the products of the factor as 64 x 64 tiles, a pair of
+// 40^3 solves took 1604 us with 8 right-hand sides, 1474 with one; now 1096
+// and 1008.
+template <int BUILD>
+__device__ __forceinline__ bool is_narrow(const Task& t) {
+  return BUILD == EB_SOLVE && t.op == T_GEMM && t.aux[0] == GEMM_NARROW;
+}
+
+static __device__ void run_trsv(const RunArgs& ra, const Task& t, double* smem, int& claim) {
   __shared__ int s_trsv_abort;
-  constexpr int LA = TRSV_LA;
+  constexpr int LA = TRSV_LA, LB = TRSV_LB;
   double* sA = smem;
   double* sB = smem + TRSV_KMAX * LA;
   const int m = t.m, n = t.n, K = t.k, K4 = (K + 3) & ~3;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   {
+    // (rows from m on stay as they are: they meet only rows of the product
+    // that are not stored)
     const double* __restrict__ X = ra.bases[t.a.base] + t.a.off;
     const int ld = t.a.ld;
     if (t.a.mode == OM_T) {
-      // A(r, k) = X[r*ld + k]: consecutive threads take consecutive k
-      for (int idx = tid; idx < TILE * K4; idx += NTHREADS) {
-        const int k = idx % K4, r = idx / K4;
-        const bool ok = r < m && k < K;
-        cp_async8_zfill(sA + k * LA + r, ok ? X + (int64_t)r * ld + k : X, ok);
-      }
+      // A(r, k) = X[r*ld + k]: a row a warp, consecutive lanes take consecutive k
+      for (int r = warp; r < m; r += NTHREADS / 32)
+        for (int k = lane; k < K4; k += 32)
+          cp_async8_zfill(sA + k * LA + r, k < K ? X + (int64_t)r * ld + k : X, k < K);
     } else {
-      for (int idx = tid; idx < TILE * K4; idx += NTHREADS) {
-        const int r = idx % TILE, k = idx / TILE;
-        const bool ok = r < m && k < K;
-        cp_async8_zfill(sA + k * LA + r, ok ? X + (int64_t)k * ld + r : X, ok);
-      }
+      for (int k = warp; k < K4; k += NTHREADS / 32)
+        for (int r = lane; r < m; r += 32)
+          cp_async8_zfill(sA + k * LA + r, k < K ? X + (int64_t)k * ld + r : X, k < K);
     }
     cp_async_commit();
   }
   if (tid == 0) {
     int abort = 0;
-    for (int w = t.cdiag; w < t.nwait && !abort; w++) {
+    // (under the dynamic schedule a narrow product is released on all its waits)
+    const int w0 = t.op == T_TRSV ? t.cdiag : (ra.dynamic ? t.nwait : 0);
+    for (int w = w0; w < t.nwait && !abort; w++) {
       const int2 wt = ra.waits[t.wait_off + w];
       int64_t spins = 0;
       unsigned ns = 16;
@@ -1091,43 +1102,55 @@ static __device__ void run_trsv(const RunArgs& ra, const Task& t, double* smem) 
   const int ldb = t.b.ld;  // B(j, k) = Xb[j*ldb + k] (x tiles, operand mode OM_T)
   double* __restrict__ C = ra.bases[t.c.base] + t.c.off;
   const int ldc = t.c.ld;
+  const int jb = tid >> 4, kb = tid & 15;  // 16 threads a column of B
   for (int j0 = 0; j0 < n; j0 += 8) {
     const int nb = min(8, n - j0);
-    for (int base = 0; base < K4 * 8; base += 4 * NTHREADS) {
-      double v[4];
+    {
+      double v[TRSV_KMAX / 16];
+      const double* __restrict__ src = Xb + (int64_t)(j0 + jb) * ldb;
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const int idx = base + tid + e * NTHREADS, k = idx % K4, j = idx / K4;
-        v[e] = (idx < K4 * 8 && k < K && j < nb) ? __ldcg(Xb + (int64_t)(j0 + j) * ldb + k) : 0.0;
-      }
+      for (int e = 0; e < TRSV_KMAX / 16; e++) v[e] = (kb + 16 * e < K && jb < nb) ? __ldcg(src + kb + 16 * e) : 0.0;
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const int idx = base + tid + e * NTHREADS, k = idx % K4, j = idx / K4;
-        if (idx < K4 * 8) sB[k * 8 + j] = v[e];
-      }
+      for (int e = 0; e < TRSV_KMAX / 16; e++) sB[jb * LB + kb + 16 * e] = v[e];
     }
     if (j0 == 0) cp_async_wait_all();
     __syncthreads();
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    if (!ra.dynamic && j0 + 8 >= n && tid == 32) claim = atomicAdd(&ra.ctl[0], 1);
     if (16 * warp < m) {
-      const double* ar = sA + 16 * warp + g;
-#pragma unroll 4
-      for (int k = 0; k < K4; k += 4) dmma16(acc, ar[(k + q) * LA], ar[(k + q) * LA + 8], sB[(k + q) * 8 + g]);
-    }
+      double acc[4][4];
 #pragma unroll
-    for (int h = 0; h < 4; h++) {
-      const int r = 16 * warp + g + ((h & 2) ? 8 : 0), j = 2 * q + (h & 1);
-      if (r < m && j < nb) {
-        double* cp = C + (int64_t)(j0 + j) * ldc + r;
-        double val = t.alpha * acc[h];
-        if (t.beta != 0.0) val += t.beta * __ldcg(cp);
-        *cp = val;
+      for (int e = 0; e < 4; e++) acc[e][0] = acc[e][1] = acc[e][2] = acc[e][3] = 0.0;
+      const double* ar = sA + 16 * warp + g;
+      const double* br = sB + g * LB;
+      for (int k0 = 0; k0 < K4; k0 += 16) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const int k = k0 + 4 * e + q;
+          if (k0 + 4 * e < K4) dmma16(acc[e], ar[k * LA], ar[k * LA + 8], br[k]);
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 4; h++) {
+        const int r = 16 * warp + g + ((h & 2) ? 8 : 0), j = 2 * q + (h & 1);
+        if (r < m && j < nb) {
+          double* cp = C + (int64_t)(j0 + j) * ldc + r;
+          double val = t.alpha * ((acc[0][h] + acc[1][h]) + (acc[2][h] + acc[3][h]));
+          if (t.cmode == CM_ATOMIC) {
+            atomicAdd(cp, val);
+          } else {
+            if (t.beta != 0.0) val += t.beta * __ldcg(cp);
+            *cp = val;
+          }
+        }
       }
     }
     __syncthreads();
   }
 }
 
+// C = alpha * M2 * (opA * opB^T), M2 = lower-triangular m x m tile (operand
+// `c` of the task holds C; M2 is described by aux: base aux[0], ld aux[1],
+// offset (aux[2] | aux[3] << 32)).
 static __device__ void run_mrow(const RunArgs& ra, const Task& t, const SmemLayout& sm) {
   const Opnd A = make_opnd(ra, t.a), B = make_opnd(ra, t.b);
   double* C = ra.bases[t.c.base] + t.c.off;
@@ -3039,41 +3062,39 @@ static __device__ void run_vec(const RunArgs& ra, const Task& t, double* smem) {
   const int i0 = t.m, i1 = t.k > 0 ? t.k : Nc, ni = max(i1 - i0, 0), tot = ni * nc;
   const int32_t* __restrict__ r = ra.relidx + ch.relptr;
   double* __restrict__ uc = WS + vbase + ch.vpos * nrhs;
-  for (int base = 0; base < tot; base += E * NTHREADS) {
-    int row[E], ui[E];
+  // EV elements per thread with their loads in flight together: the planner's
+  // chunks (2048 elements) take one pass, two L2 round trips in an extraction
+  // and one in an addition, whose values need not wait for the indices
+  constexpr int EV = 16;
+  for (int base = 0; base < tot; base += EV * NTHREADS) {
+    int row[EV], col[EV];
+    double v[EV];
 #pragma unroll
-    for (int e = 0; e < E; e++) {
+    for (int e = 0; e < EV; e++) {
       const int idx = base + threadIdx.x + e * NTHREADS;
-      const int i = i0 + idx % max(ni, 1), j = j0 + idx / max(ni, 1);
+      const int j = idx / max(ni, 1), i = i0 + idx - j * ni;
+      col[e] = j0 + j;
       row[e] = (idx < tot) ? __ldg(r + i) : -1;
-      ui[e] = i + j * Nc;
+      if (mode == VEC_ADD) v[e] = (idx < tot) ? __ldcg(uc + i + (int64_t)(j0 + j) * Nc) : 0.0;
     }
+    auto entry = [&](int e) {
+      return row[e] < f.nn ? xp + row[e] + (int64_t)col[e] * ldx : up + (row[e] - f.nn) + (int64_t)col[e] * f.na;
+    };
     if (mode == VEC_ADD) {
       // rows of one child are distinct, but other children add into the
       // same rows at the same time: atomic adds
-      double v[E];
 #pragma unroll
-      for (int e = 0; e < E; e++) v[e] = row[e] >= 0 ? __ldcg(uc + ui[e]) : 0.0;
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        if (row[e] < 0) continue;
-        const int j = j0 + (base + threadIdx.x + e * NTHREADS) / max(ni, 1);
-        double* dst = row[e] < f.nn ? xp + row[e] + (int64_t)j * ldx : up + (row[e] - f.nn) + (int64_t)j * f.na;
-        atomicAdd(dst, v[e]);
-      }
+      for (int e = 0; e < EV; e++)
+        if (row[e] >= 0) atomicAdd(entry(e), v[e]);
       continue;
     }
-    double v[E];
 #pragma unroll
-    for (int e = 0; e < E; e++) {
-      const int j = j0 + (base + threadIdx.x + e * NTHREADS) / max(ni, 1);
-      v[e] = row[e] < 0 ? 0.0
-                        : (row[e] < f.nn ? __ldcg(xp + row[e] + (int64_t)j * ldx)
-                                         : __ldcg(up + (row[e] - f.nn) + (int64_t)j * f.na));
+    for (int e = 0; e < EV; e++) v[e] = row[e] < 0 ? 0.0 : __ldcg(entry(e));
+#pragma unroll
+    for (int e = 0; e < EV; e++) {
+      const int idx = base + threadIdx.x + e * NTHREADS;
+      if (row[e] >= 0) uc[i0 + idx - (col[e] - j0) * ni + (int64_t)col[e] * Nc] = v[e];
     }
-#pragma unroll
-    for (int e = 0; e < E; e++)
-      if (row[e] >= 0) uc[ui[e]] = v[e];
   }
 }
 
@@ -3299,7 +3320,8 @@ static_assert(8 * SUB_NJ * SUB_LD <= ENGINE_SMEM_BASE_DOUBLES, "bundle fronts ex
 // it, a launch of the FP64 sweeps measured 17-60 % slower at 40^3, although
 // no tcgen05 instruction ran; with the register-resident Householder panels
 // in it, cholesky + projected_inverse took 12.17 ms there against 11.99
-// without them.
+// without them; with the solve tasks, 10.37 against 10.35 (97^2 with extra
+// edges 2.22 against 2.20).
 template <int BUILD>
 __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
   constexpr bool TC = BUILD == EB_TCGEN05;
@@ -3398,7 +3420,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
           if (lane == 0 && ra.trace) ra.trace[4 * (int64_t)ti] = global_ns();
           __syncwarp();
           int timed_out = 0;
-          const int npre = ((s_t.op == T_POTRF && s_t.k > 0) || s_t.op == T_TRSV) ? (int)s_t.cdiag : (int)s_t.nwait;
+          const int npre = ((s_t.op == T_POTRF && s_t.k > 0) || s_t.op == T_TRSV) ? (int)s_t.cdiag
+                           : is_narrow<BUILD>(s_t) ? 0 : (int)s_t.nwait;
           for (int w0 = 0; w0 < npre; w0 += 32) {
             if (w0 + lane < npre) {
               const int2 wt = ra.waits[s_t.wait_off + w0 + lane];
@@ -3438,7 +3461,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
     const int ti = s_task;
     const Task& t = s_t;
     claim = -1;
-    switch (t.op) {
+    switch (is_narrow<BUILD>(t) ? T_TRSV : t.op) {
       case T_GEMM:
       case T_LA: run_gemm_or_la<TC>(ra, t, sm, ts, claim); break;
       case T_MROW: run_mrow(ra, t, sm); break;
@@ -3450,8 +3473,14 @@ __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
       case T_PSUBTREE: run_subtrees(ra, t, smem); break;
       case T_EXTRACT: run_extract(ra, t, smem); break;
       case T_COPY: run_copy(ra, t); break;
-      case T_VEC: run_vec(ra, t, smem); break;
-      case T_TRSV: run_trsv(ra, t, smem); break;
+      case T_VEC:
+        if (BUILD == EB_SOLVE) run_vec(ra, t, smem);
+        else if (threadIdx.x == 0) atomicCAS(&ra.ctl[1], 0, DE_BAD_TASK);
+        break;
+      case T_TRSV:
+        if (BUILD == EB_SOLVE) run_trsv(ra, t, smem, claim);
+        else if (threadIdx.x == 0) atomicCAS(&ra.ctl[1], 0, DE_BAD_TASK);
+        break;
       case T_QL:
         if (BUILD == EB_PANELS) run_ql(ra, t, smem);
         else if (threadIdx.x == 0) atomicCAS(&ra.ctl[1], 0, DE_BAD_TASK);

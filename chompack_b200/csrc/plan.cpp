@@ -156,6 +156,7 @@ Program* build_host_program(chb_plan* plan, int op, int64_t k, int flags) {
   for (const Task& t : prog->tasks) {
     if (t.op == T_QL || t.op == T_TRSV) prog->smem_doubles = ENGINE_SMEM_DOUBLES;  // Householder panels, step operands
     if (t.op == T_QL) prog->panels = true;
+    if (t.op == T_VEC || t.op == T_TRSV) prog->solve = true;
   }
   // Every sweep runs in static list order by default: a CTA already waits on
   // its next task, while a task released under the dynamic schedule is
@@ -247,6 +248,7 @@ int run_program(chb_plan* plan, Program* prog, void* work, size_t work_bytes, do
   // accumulators when the plan asks for it
   ra.tmem = prog->tf32_tiles && tf32_tcgen05(*plan) ? 1 : 0;
   ra.panels = prog->panels ? 1 : 0;
+  ra.solve = prog->solve ? 1 : 0;
   ra.ldb = run_ldb;
   ra.alpha = run_alpha;
   // The plan's schedule, else CHB_SCHEDULE (static | dynamic), else static.

@@ -38,6 +38,7 @@ struct Program {
   int64_t ncounters = 0;   // tasks + groups
   int64_t ws_doubles = 0;  // doubles of workspace (update matrices + scratch)
   bool panels = false;                          // has Householder panels (T_QL tasks)
+  bool solve = false;                           // has solve tasks (T_VEC, T_TRSV)
   int smem_doubles = ENGINE_SMEM_BASE_DOUBLES;  // dynamic shared memory per CTA
   bool tf32_tiles = false;      // some GEMM tile computes in TF32 (one product)
   IoSpec io;                    // streaming of the values (set before building)
