@@ -1,5 +1,6 @@
 // Task-graph engine shared by the host planner (plan.cpp) and the device
-// executor (engine_kernel.cuh, built by engine.cu, engine_tc.cu, engine_ql.cu).
+// executor (engine_kernel.cuh, built by engine.cu, engine_tc.cu,
+// engine_ql.cu, engine_solve.cu).
 //
 // Every numeric sweep is compiled on the host into a list of tile tasks in a
 // topological order.  One persistent kernel executes the list: each CTA

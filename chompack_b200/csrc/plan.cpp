@@ -158,7 +158,7 @@ Program* build_host_program(chb_plan* plan, int op, int64_t k, int flags) {
     if (t.op == T_QL) prog->panels = true;
     if (t.op == T_VEC || t.op == T_TRSV) prog->solve = true;
   }
-  // Every sweep runs in static list order by default: a CTA already waits on
+  // Sweeps run in static list order by default: a CTA already waits on
   // its next task, while a task released under the dynamic schedule is
   // published, found and claimed, about 7 us a hop when the CTAs are idle.
   // Static against dynamic: unfactored completion on 3-D 40^3 12.5 / 14.0 ms
@@ -166,6 +166,12 @@ Program* build_host_program(chb_plan* plan, int op, int64_t k, int flags) {
   // hessian (unfactored) 31.9 / 35.7 and 1.8 / 2.9, projected_inverse 5.5 /
   // 5.7 and 0.95 / 1.01, on 2-D 1000^2 9.7 / 12.3, and under a scratch limit
   // 10.8 / 13.7; no sweep at any measured size was faster dynamically.
+  // Sweeps on host-resident values run dynamically: a CTA in list order
+  // waits on a chunk of the values that has not arrived, while tasks of
+  // those that have are ready.  Static against dynamic, cholesky and
+  // projected_inverse on 3-D 40^3 18.5 / 13.8 and 18.1 / 13.9 ms, on 24^3 2.11
+  // / 2.06 and 2.42 / 2.05, on 2-D 400^2 9.1 / 7.0 and 9.4 / 6.8.
+  prog->static_default = !prog->io.in && !prog->io.out;
   Program* p = prog.get();
   plan->progs[key] = std::move(prog);
   return p;
@@ -251,9 +257,11 @@ int run_program(chb_plan* plan, Program* prog, void* work, size_t work_bytes, do
   ra.solve = prog->solve ? 1 : 0;
   ra.ldb = run_ldb;
   ra.alpha = run_alpha;
-  // The plan's schedule, else CHB_SCHEDULE (static | dynamic), else static.
+  // The plan's schedule, else CHB_SCHEDULE (static | dynamic), else the
+  // program's default.
   static const char* sched = std::getenv("CHB_SCHEDULE");
-  bool want_static = true;
+  bool want_static = prog->static_default;
+  if (sched && std::strcmp(sched, "static") == 0) want_static = true;
   if (sched && std::strcmp(sched, "dynamic") == 0) want_static = false;
   if (plan->schedule >= 0) want_static = plan->schedule == 1;
   const bool dynamic = !want_static && prog->d_npend && prog->d_ready0;

@@ -37,6 +37,7 @@ struct Program {
   std::vector<int2> waits;
   int64_t ncounters = 0;   // tasks + groups
   int64_t ws_doubles = 0;  // doubles of workspace (update matrices + scratch)
+  bool static_default = true;                   // static list order unless the plan or CHB_SCHEDULE says otherwise
   bool panels = false;                          // has Householder panels (T_QL tasks)
   bool solve = false;                           // has solve tasks (T_VEC, T_TRSV)
   int smem_doubles = ENGINE_SMEM_BASE_DOUBLES;  // dynamic shared memory per CTA
