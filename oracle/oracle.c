@@ -719,3 +719,68 @@ double orc_dot(int64_t nsn, const int64_t* snptr, const int64_t* sncolptr, const
 int orc_update_factor(const int64_t* r, int nn, int na, double* u, int N, const double* f, int ldf, double* C) {
   return update_factor_o(r, nn, na, u, N, f, ldf, C);
 }
+
+/* Product form of I + V diag(a) V^T (pfcholesky.c:52-136): factor i is the
+ * lower triangular L_i with diagonal l_i and entries v_r b_c below it
+ * (r > c), n x k column-major arrays with leading dimension n. */
+
+/* x := L_i^{-1} x, or L_i^{-T} x */
+static void pf_solve(int64_t n, int trans, const double* v, const double* l, const double* b, double* x) {
+  double s = 0.0;
+  if (!trans)
+    for (int64_t r = 0; r < n; r++) {
+      x[r] = (x[r] - v[r] * s) / l[r];
+      s += b[r] * x[r];
+    }
+  else
+    for (int64_t r = n - 1; r >= 0; r--) {
+      x[r] = (x[r] - b[r] * s) / l[r];
+      s += v[r] * x[r];
+    }
+}
+
+/* x := L_i x, or L_i^T x */
+static void pf_multiply(int64_t n, int trans, const double* v, const double* l, const double* b, double* x) {
+  double s = 0.0;
+  if (!trans)
+    for (int64_t r = 0; r < n; r++) {
+      const double y = x[r];
+      x[r] = l[r] * y + v[r] * s;
+      s += b[r] * y;
+    }
+  else
+    for (int64_t r = n - 1; r >= 0; r--) {
+      const double y = x[r];
+      x[r] = l[r] * y + b[r] * s;
+      s += v[r] * y;
+    }
+}
+
+/* The factors of I + V diag(a) V^T; column i of V becomes
+ * (L_1 ... L_i)^{-1} v_i.  Returns -1 where 1 - alpha v^2 is not positive. */
+int orc_pfchol(int64_t n, int64_t k, const double* a, double* V, double* L, double* B) {
+  for (int64_t i = 0; i < k; i++) {
+    double *v = V + i * n, *l = L + i * n, *b = B + i * n, alpha = -a[i];
+    for (int64_t r = 0; r < n; r++) {
+      const double d = 1.0 - alpha * v[r] * v[r];
+      if (!(d > 0.0)) return -1;
+      l[r] = sqrt(d);
+      b[r] = -alpha * v[r] / l[r];
+      alpha += b[r] * b[r];
+    }
+    for (int64_t c = i + 1; c < k; c++) pf_solve(n, 0, v, l, b, V + c * n);
+  }
+  return 0;
+}
+
+/* U (n x m) := (L_1 ... L_k)^{-1} U or its transpose's (solve), L_1 ... L_k U
+ * or (L_1 ... L_k)^T U (!solve) */
+void orc_pfapply(int64_t n, int64_t k, int64_t m, int solve, int trans, const double* V, const double* L,
+                 const double* B, double* U) {
+  for (int64_t j = 0; j < m; j++)
+    for (int64_t q = 0; q < k; q++) {
+      const int64_t i = n * ((solve != 0) == (trans != 0) ? k - 1 - q : q);
+      if (solve) pf_solve(n, trans, V + i, L + i, B + i, U + j * n);
+      else pf_multiply(n, trans, V + i, L + i, B + i, U + j * n);
+    }
+}

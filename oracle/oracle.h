@@ -44,4 +44,9 @@ int orc_update_factor(const int64_t* r, int nn, int na, double* u, int N, const 
 double orc_dot(int64_t nsn, const int64_t* snptr, const int64_t* sncolptr, const int64_t* blkptr,
                const double* x, const double* y);
 
+int orc_pfchol(int64_t n, int64_t k, const double* a, double* V, double* L, double* B);
+
+void orc_pfapply(int64_t n, int64_t k, int64_t m, int solve, int trans, const double* V, const double* L,
+                 const double* B, double* U);
+
 #endif

@@ -39,6 +39,10 @@ def lib():
         _lib.orc_trsm.restype = None
         _lib.orc_dot.argtypes = [i64, pi, pi, pi, pd, pd]
         _lib.orc_dot.restype = ctypes.c_double
+        _lib.orc_pfchol.argtypes = [i64, i64, pd, pd, pd, pd]
+        _lib.orc_pfchol.restype = ctypes.c_int
+        _lib.orc_pfapply.argtypes = [i64, i64, i64, ctypes.c_int, ctypes.c_int, pd, pd, pd, pd]
+        _lib.orc_pfapply.restype = None
     return _lib
 
 
@@ -137,3 +141,33 @@ def dot(symb, x, y):
     a = [_i(np.asarray(getattr(symb, nm))) for nm in ("snptr", "sncolptr", "blkptr")]
     keep += [t[0] for t in a]
     return lib().orc_dot(int(symb.Nsn), a[0][1], a[1][1], a[2][1], _d(x), _d(y))
+
+
+def _dF(a):
+    assert a.dtype == np.float64 and a.flags["F_CONTIGUOUS"]
+    return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
+
+
+def pfchol(a, V):
+    """(L, B, info) of the product-form factor of I + V diag(a) V^T; V (n x k,
+    Fortran-ordered) is overwritten."""
+    n, k = V.shape
+    L, B = np.zeros((n, k), order="F"), np.zeros((n, k), order="F")
+    info = lib().orc_pfchol(n, k, _d(np.ascontiguousarray(a, dtype=np.float64)), _dF(V), _dF(L), _dF(B))
+    return L, B, info
+
+
+def _pfapply(solve, V, L, B, U, trans):
+    n, k = V.shape
+    lib().orc_pfapply(n, k, U.size // n, solve, 1 if trans == 'T' else 0, _dF(V), _dF(L), _dF(B), _dF(U))
+    return U
+
+
+def pftrsm(V, L, B, U, trans='N'):
+    """U := (L_1 ... L_k)^{-1} U ('N') or (L_k^T ... L_1^T)^{-1} U ('T')."""
+    return _pfapply(1, V, L, B, U, trans)
+
+
+def pftrmm(V, L, B, U, trans='N'):
+    """U := L_1 ... L_k U ('N') or L_k^T ... L_1^T U ('T')."""
+    return _pfapply(0, V, L, B, U, trans)

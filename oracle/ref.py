@@ -9,13 +9,22 @@ does (src/C/cbase.c: cchol :187-284, cllt :298-390, cprojected_inverse
 :106-174): int_t is Py_ssize_t (int64), workspaces are sized from
 symb.memory, and the U list of hessian is NULL-terminated.
 
+Where those kernels are not built (the reference's sources are absent), the
+functions below run the C restatement of the same sweeps instead
+(oracle/oracle.py, which tests/test_oracle.py holds against the reference);
+source() says which of the two answers.  available() and lib() are about the
+reference's own kernels only: a timing of the reference needs them.
+
 All arrays are numpy; `symb` is any object with the reference's symbolic
 attributes (chompack_b200.symbolic qualifies: its arrays are bit-identical).
 """
 import ctypes
+import functools
 import os
 
 import numpy as np
+
+from oracle import oracle
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB = os.path.join(HERE, "_ref", "libchompack_ref.so")
@@ -25,6 +34,19 @@ _lib = None
 
 def available():
     return os.path.exists(LIB)
+
+
+def source():
+    """What the functions of this module run."""
+    return "reference C kernels (oracle/_ref)" if available() else "C restatement (oracle/oracle.c)"
+
+
+def _or_restated(fn):
+    """fn on the reference's kernels, or its namesake of oracle/oracle.py."""
+    @functools.wraps(fn)
+    def call(*args, **kwargs):
+        return (fn if available() else getattr(oracle, fn.__name__))(*args, **kwargs)
+    return call
 
 
 def lib():
@@ -102,6 +124,7 @@ class _Sym(object):
                 self.blkptr)
 
 
+@_or_restated
 def cholesky(symb, blkval):
     """In-place reference cholesky on a float64 numpy blkval; returns info."""
     s = _Sym(symb)
@@ -109,6 +132,7 @@ def cholesky(symb, blkval):
     return lib().cholesky(*s.common(), _d(blkval), fws, upd, usz)
 
 
+@_or_restated
 def llt(symb, blkval):
     s = _Sym(symb)
     fws, upd, usz = s.ws()
@@ -116,18 +140,21 @@ def llt(symb, blkval):
     return 0
 
 
+@_or_restated
 def projected_inverse(symb, blkval):
     s = _Sym(symb)
     fws, upd, usz = s.ws()
     return lib().projected_inverse(*s.common(), _d(blkval), fws, upd, usz)
 
 
+@_or_restated
 def completion(symb, blkval, factored_updates=True):
     s = _Sym(symb)
     fws, upd, usz = s.ws()
     return lib().completion(*s.common(), _d(blkval), fws, upd, usz, 1 if factored_updates else 0)
 
 
+@_or_restated
 def hessian(symb, lblkval, yblkval, ublkvals, adj=False, inv=False, factored_updates=True):
     """Reference hessian on a list of U blkvals (each updated in place).
     adj=None applies the full Hessian: two passes with adj toggled, as
@@ -147,6 +174,7 @@ def hessian(symb, lblkval, yblkval, ublkvals, adj=False, inv=False, factored_upd
     return info
 
 
+@_or_restated
 def trsm(symb, blkval, B, alpha=1.0, trans='N', nrhs=None, offsetB=0, ldB=None):
     """Reference trsm on a column-major numpy B (flattened, Fortran order)."""
     s = _Sym(symb)
@@ -172,6 +200,7 @@ def trsm(symb, blkval, B, alpha=1.0, trans='N', nrhs=None, offsetB=0, ldB=None):
     return B
 
 
+@_or_restated
 def dot(symb, x, y):
     s = _Sym(symb)
     nsn = ctypes.c_int64(s.nsn)
@@ -179,8 +208,10 @@ def dot(symb, x, y):
 
 
 def set_threads(n):
-    """Thread count of the OpenBLAS the reference kernels are linked against."""
-    lib()
+    """Thread count of the OpenBLAS the reference kernels are linked against
+    (the restatement is single-threaded)."""
+    if not available():
+        return False
     import glob
     import scipy
     d = os.path.realpath(os.path.join(os.path.dirname(scipy.__file__), "..", "scipy.libs"))
@@ -205,6 +236,7 @@ def _dF(a):
     return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
 
 
+@_or_restated
 def pfchol(a, V):
     """Returns (L, B, info) of dpftrf on V (modified in place)."""
     assert V.flags["F_CONTIGUOUS"] and V.dtype == np.float64
@@ -227,11 +259,13 @@ def _pf_columns(fn, V, L, B, U, trans):
     return U
 
 
+@_or_restated
 def pftrsm(V, L, B, U, trans='N'):
     """U := (L_1 ... L_k)^{-1} U ('N') or (L_k^T ... L_1^T)^{-1} U ('T')."""
     return _pf_columns(lib().dpfsv, V, L, B, U, trans)
 
 
+@_or_restated
 def pftrmm(V, L, B, U, trans='N'):
     """U := L_1 ... L_k U ('N') or L_k^T ... L_1^T U ('T')."""
     return _pf_columns(lib().dpfmv, V, L, B, U, trans)
