@@ -1328,176 +1328,7 @@ __device__ __forceinline__ void potrf_syrk_tile(double* sL, int jp, int r0, int 
   if (r + 8 >= c + 1) sL[(c + 1) * LD + r + 8] = ac[3];
 }
 
-// Cholesky of a 16 x 16 diagonal block sL (factor; else the block already
-// holds L) and its inverse sM (lower part written), by one warp, in two
-// 8-column groups (only the first with cols <= 8, where the rest of the
-// block is the identity).
-// Every lane holds the group's 8 x 8 block and factors it for itself, so the
-// chain from pivot to pivot is rsqrt -> multiply -> FMA with no exchange;
-// beside it lane i reduces row i of the group's columns (the 8 rows of the
-// block, then the 8 rows below) and lane c afterwards forms column c of the
-// block's inverse.  The second diagonal 8 x 8 block takes its rank-8 update,
-// and the block below the inverse's diagonal its two products, by MMAs.
-// One lane per row with every pivot column broadcast through shared memory
-// took 300 cycles a pivot on an idle SM: 19.2k for the 64 of a tile, and 6.4k
-// for its four inverses; this takes 13.8k for both (with library rsqrt()
-// 16.7k), and the whole 64 x 64 task 22k instead of 41.8k cycles.
-// Returns the block's first non-positive pivot (zero pivot when !factor), or
-// -1; such a pivot is taken as 1.
-
-// 1 / sqrt(d) for d in [1e-300, 1e300]: the hardware's approximation (about
-// 20 bits) and one third-order step, y + y e (1/2 + 3/8 e) with
-// e = 1 - d y^2, whose error is about 5/16 e^3.  54 cycles in a dependent
-// chain against 66 for rsqrt(), and no branch.
-__device__ __forceinline__ double rsqrt_normal(double d) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double e = fma(-(d * y), y, 1.0);
-  return fma(fma(e, 0.375, 0.5), y * e, y);
-}
-
-// The pivots of an 8 x 8 block held by every lane (a, lower part), with the
-// lane's row x beside them; r = 1 / L(j, j).  Returns false, with results to
-// be thrown away, when a pivot lies outside [1e-300, 1e300].
-__device__ __forceinline__ bool potrf_pivots8(double (&a)[8][8], double (&x)[8], double (&r)[8]) {
-  bool ok = true;
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    // the high words of 1e-300 and 1e300: positive, finite, no NaN between them
-    ok = ok && (unsigned)(__double2hiint(a[j][j]) - 0x01A56E20) < 0x7E37E43Cu - 0x01A56E20u;
-    r[j] = rsqrt_normal(a[j][j]);
-    x[j] *= r[j];
-#pragma unroll
-    for (int i = j + 1; i < 8; i++) a[j][i] *= r[j];
-#pragma unroll
-    for (int c = j + 1; c < 8; c++) {
-#pragma unroll
-      for (int i = c; i < 8; i++) a[c][i] = fma(-a[j][i], a[j][c], a[c][i]);
-      x[c] = fma(-x[j], a[j][c], x[c]);
-    }
-  }
-  return ok;
-}
-
-// The same for any pivots, in place in shared memory (rows b0 .. b0 + nr, a
-// lane each): a non-positive one is taken as 1.  Returns the first, or -1.
-template <int LD>
-__device__ __forceinline__ int potrf_pivots8_any(double* sL, int b0, int nr) {
-  const int lane = threadIdx.x & 31;
-  int bad = -1;
-#pragma unroll 1
-  for (int j = 0; j < 8; j++) {
-    double* const col = sL + (b0 + j) * LD + b0;
-    const double d = col[j];
-    const bool np = !(d > 0.0);
-    if (np && bad < 0) bad = j;
-    const double rs = rsqrt(np ? 1.0 : d), v = lane < nr ? col[lane] * rs : 0.0;
-    __syncwarp();
-    if (lane >= j && lane < nr) col[lane] = lane == j && np ? 1.0 : v;
-    __syncwarp();
-#pragma unroll 1
-    for (int c = j + 1; c < 8; c++)
-      if (lane >= c && lane < nr) sL[(b0 + c) * LD + b0 + lane] = fma(-v, col[c], sL[(b0 + c) * LD + b0 + lane]);
-    __syncwarp();
-  }
-  return bad;
-}
-
-template <int LD, int LDM>
-__device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw, bool factor, int cols = 16) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, c8 = lane & 7;
-  int first_bad = -1;
-#pragma unroll 1
-  for (int h = 0; h < (cols > 8 ? 2 : 1); h++) {
-    const int b0 = 8 * h;
-    double a[8][8], r[8];  // a[c][i]: entry (i, c), i >= c
-    // row b0 + (lane mod 16): of the block, or below it (h = 0)
-    const int row = b0 + (h == 0 ? (lane & 15) : c8);
-    double x[8];
-    auto load = [&] {
-#pragma unroll
-      for (int c = 0; c < 8; c++) {
-#pragma unroll
-        for (int i = c; i < 8; i++) a[c][i] = sL[(b0 + c) * LD + b0 + i];
-        x[c] = sL[(b0 + c) * LD + row];
-      }
-    };
-    load();
-    if (factor) {
-      const int nr = h == 0 ? 16 : 8;
-      const bool ok = potrf_pivots8(a, x, r);
-      __syncwarp();
-      if (ok) {
-        if (lane < nr) {
-#pragma unroll
-          for (int c = 0; c < 8; c++)
-            if (lane >= c) sL[(b0 + c) * LD + row] = x[c];
-        }
-      } else {
-        const int bad = potrf_pivots8_any<LD>(sL, b0, nr);
-        if (bad >= 0 && first_bad < 0) first_bad = 8 * h + bad;
-        load();
-#pragma unroll
-        for (int j = 0; j < 8; j++) r[j] = 1.0 / a[j][j];
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const bool bad = a[j][j] == 0.0;
-        first_bad = (bad && first_bad < 0) ? 8 * h + j : first_bad;
-        r[j] = 1.0 / (bad ? 1.0 : a[j][j]);
-      }
-    }
-    // column c8 of the inverse, right-looking: as soon as M(l, c) is known it
-    // is added into the partial sums of the later rows
-    double m[8], t[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) t[i] = 0.0;
-#pragma unroll
-    for (int l = 0; l < 8; l++) {
-      m[l] = l == c8 ? r[l] : (l > c8 ? -r[l] * t[l] : 0.0);
-#pragma unroll
-      for (int i = l + 1; i < 8; i++) t[i] = fma(a[l][i], m[l], t[i]);
-    }
-    if (lane < 8) {
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-        if (i >= c8) sM[(b0 + c8) * LDM + b0 + i] = m[i];
-    }
-    __syncwarp();
-    if (factor && h == 0) {
-      // the second diagonal block: A(r, c) -= sum_k L(r, k) L(c, k), lower part
-      const int rr = 8 + g, cc = 8 + 2 * q;
-      double v[2] = {sL[cc * LD + rr], sL[(cc + 1) * LD + rr]};
-#pragma unroll
-      for (int k = 0; k < 8; k += 4) {
-        const double w = sL[(k + q) * LD + rr];
-        dmma8(v, -w, w);
-      }
-      if (rr >= cc) sL[cc * LD + rr] = v[0];
-      if (rr >= cc + 1) sL[(cc + 1) * LD + rr] = v[1];
-      __syncwarp();
-    }
-  }
-  if (cols <= 8) {  // the second half is the identity, as L's is
-    if (lane < 8) sM[(8 + lane) * LDM + 8 + lane] = 1.0;
-    return first_bad;
-  }
-  // M21 = -M22 (L21 M11)
-  double v[2] = {0.0, 0.0};
-#pragma unroll
-  for (int k = 0; k < 8; k += 4)
-    dmma8(v, sL[(k + q) * LD + 8 + g], sM[g * LDM + k + q]);
-  sTw[16 * q + g] = v[0];  // column-major
-  sTw[16 * q + 8 + g] = v[1];
-  __syncwarp();
-  v[0] = v[1] = 0.0;
-#pragma unroll
-  for (int k = 0; k < 8; k += 4) dmma8(v, -sM[(8 + k + q) * LDM + 8 + g], sTw[8 * g + k + q]);
-  sM[2 * q * LDM + 8 + g] = v[0];
-  sM[(2 * q + 1) * LDM + 8 + g] = v[1];
-  return first_bad;
-}
+#include "block16.cuh"
 
 // Block row I of the inverse, column tiles of 8 columns: first the products
 // T = L(I, :I) M(:I, tile) (K = 16 I) in the tile's place in sM, then, once
