@@ -43,7 +43,8 @@ __device__ __forceinline__ int potrf_pivots8(double (&a)[8][8], double (&x)[8], 
 // took 300 cycles a pivot on an idle SM: 19.2k for the 64 of a tile, and 6.4k
 // for its four inverses; this takes 16.7k for both.
 // Returns the block's first non-positive pivot (zero pivot when !factor), or
-// -1; such a pivot is taken as 1.
+// -1; such a pivot is taken as 1.  Without factor, sM may be sL: the inverse
+// takes the block's place.
 template <int LD, int LDM>
 __device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw, bool factor, int cols = 16) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, c8 = lane & 7;
@@ -77,6 +78,7 @@ __device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw
         first_bad = (bad && first_bad < 0) ? 8 * h + j : first_bad;
         r[j] = 1.0 / (bad ? 1.0 : a[j][j]);
       }
+      __syncwarp();  // in place: every lane has read the block
     }
     // column c8 of the inverse, right-looking: as soon as M(l, c) is known it
     // is added into the partial sums of the later rows

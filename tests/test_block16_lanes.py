@@ -1,6 +1,6 @@
 """The warp routine of the 16 x 16 diagonal blocks on the CPU (see
 block16_lanes.cpp): pivots over the whole range of the type, a failing
-pivot."""
+pivot, the inverse in place of the block."""
 import ctypes
 import os
 import subprocess
@@ -61,3 +61,14 @@ def test_failing_pivot(block16, bad):
     A[bad, bad] = -1.0
     L, M, info = block16(A, True)
     assert info == bad and L[bad, bad] == 1.0
+
+
+@pytest.mark.parametrize("cols", [3, 8, 11, 16])
+@pytest.mark.parametrize("down", [False, True])
+def test_inverse_in_place(block16, cols, down):
+    L = np.linalg.cholesky(spd(cols, 40 + cols))
+    _, M, info = block16(L, False, cols, down)
+    assert info == -1
+    assert np.allclose(np.tril(M) @ L, np.eye(16), rtol=0, atol=1e-13)
+    _, Mi, info = block16(L, False, cols, down, in_place=True)
+    assert info == -1 and np.array_equal(np.tril(Mi), np.tril(M))
