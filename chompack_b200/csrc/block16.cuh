@@ -37,8 +37,11 @@ __device__ __forceinline__ int potrf_pivots8(double (&a)[8][8], double (&x)[8], 
 // chain from pivot to pivot is rsqrt -> multiply -> FMA with no exchange;
 // beside it lane i reduces row i of the group's columns (the 8 rows of the
 // block, then the 8 rows below) and lane c afterwards forms column c of the
-// block's inverse.  The second diagonal 8 x 8 block takes its rank-8 update,
-// and the block below the inverse's diagonal its two products, by MMAs.
+// inverse by substitution, the first eight columns in two halves.  (As
+// M21 = -M22 (L21 M11) the lower left block would lose what the conditions
+// of both diagonal blocks multiply to.)  The second diagonal 8 x 8 block takes
+// its rank-8 update, and the columns of the inverse the product between their
+// halves, by MMAs.
 // One lane per row with every pivot column broadcast through shared memory
 // took 300 cycles a pivot on an idle SM: 19.2k for the 64 of a tile, and 6.4k
 // for its four inverses; this takes 16.7k for both.
@@ -80,23 +83,34 @@ __device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw
       }
       __syncwarp();  // in place: every lane has read the block
     }
-    // column c8 of the inverse, right-looking: as soon as M(l, c) is known it
-    // is added into the partial sums of the later rows
+    // column b0 + first of the inverse, right-looking: as soon as M(l, c) is
+    // known it is added into the partial sums of the later rows
+    const int first = h == 0 ? c8 : (lane & 15) - 8;
     double m[8], t[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) t[i] = 0.0;
+    for (int i = 0; i < 8; i++) t[i] = first < 0 ? sTw[8 * c8 + i] : 0.0;
 #pragma unroll
     for (int l = 0; l < 8; l++) {
-      m[l] = l == c8 ? r[l] : (l > c8 ? -r[l] * t[l] : 0.0);
+      m[l] = l == first ? r[l] : (l > first ? -r[l] * t[l] : 0.0);
 #pragma unroll
       for (int i = l + 1; i < 8; i++) t[i] = fma(a[l][i], m[l], t[i]);
     }
-    if (lane < 8) {
+    if (lane < (h == 0 ? 8 : 16)) {
 #pragma unroll
       for (int i = 0; i < 8; i++)
-        if (i >= c8) sM[(b0 + c8) * LDM + b0 + i] = m[i];
+        if (i >= first) sM[(b0 + first) * LDM + b0 + i] = m[i];
     }
     __syncwarp();
+    if (h == 0 && cols > 8) {
+      // what the first eight columns of the inverse start the second half
+      // with: L21 M11, column-major
+      double v[2] = {0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < 8; k += 4) dmma8(v, sL[(k + q) * LD + 8 + g], sM[g * LDM + k + q]);
+      sTw[16 * q + g] = v[0];
+      sTw[16 * q + 8 + g] = v[1];
+      __syncwarp();
+    }
     if (factor && h == 0) {
       // the second diagonal block: A(r, c) -= sum_k L(r, k) L(c, k), lower part
       const int rr = 8 + g, cc = 8 + 2 * q;
@@ -111,22 +125,6 @@ __device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw
       __syncwarp();
     }
   }
-  if (cols <= 8) {  // the second half is the identity, as L's is
-    if (lane < 8) sM[(8 + lane) * LDM + 8 + lane] = 1.0;
-    return first_bad;
-  }
-  // M21 = -M22 (L21 M11)
-  double v[2] = {0.0, 0.0};
-#pragma unroll
-  for (int k = 0; k < 8; k += 4)
-    dmma8(v, sL[(k + q) * LD + 8 + g], sM[g * LDM + k + q]);
-  sTw[16 * q + g] = v[0];  // column-major
-  sTw[16 * q + 8 + g] = v[1];
-  __syncwarp();
-  v[0] = v[1] = 0.0;
-#pragma unroll
-  for (int k = 0; k < 8; k += 4) dmma8(v, -sM[(8 + k + q) * LDM + 8 + g], sTw[8 * g + k + q]);
-  sM[2 * q * LDM + 8 + g] = v[0];
-  sM[(2 * q + 1) * LDM + 8 + g] = v[1];
+  if (cols <= 8 && lane < 8) sM[(8 + lane) * LDM + 8 + lane] = 1.0;  // the second half is the identity, as L's is
   return first_bad;
 }

@@ -1,6 +1,6 @@
 """The warp routine of the 16 x 16 diagonal blocks on the CPU (see
 block16_lanes.cpp): pivots over the whole range of the type, a failing
-pivot, the inverse in place of the block."""
+pivot, the inverse in place of the block and its residual."""
 import ctypes
 import os
 import subprocess
@@ -72,3 +72,19 @@ def test_inverse_in_place(block16, cols, down):
     assert np.allclose(np.tril(M) @ L, np.eye(16), rtol=0, atol=1e-13)
     _, Mi, info = block16(L, False, cols, down, in_place=True)
     assert info == -1 and np.array_equal(np.tril(Mi), np.tril(M))
+
+
+@pytest.mark.parametrize("seed", range(8))
+def test_inverse_residual(block16, seed):
+    # ill-conditioned 8 x 8 diagonal blocks (9e5), L21 = K2 Z K1
+    rng = np.random.default_rng(seed)
+    c, s = np.cos(0.3), np.sin(0.3)
+    K1, K2 = ((np.eye(8) - c * np.tril(np.ones((8, 8)), -1)) * s ** np.arange(8) * (1 + 0.1 * rng.random((8, 8)))
+              for _ in range(2))
+    L = np.block([[K1, np.zeros((8, 8))], [K2 @ rng.standard_normal((8, 8)) @ K1, K2]])
+    _, M, info = block16(L, False)
+    assert info == -1
+    L, M = L.astype(np.longdouble), np.tril(M).astype(np.longdouble)
+    # column substitution: |L M - I| <= gamma_n |L| |M|, with a rounded
+    # reciprocal and a product in place of a division
+    assert np.all(np.abs(L @ M - np.eye(16)) <= 20 * U * (np.abs(L) @ np.abs(M)))
