@@ -47,8 +47,8 @@ __device__ __forceinline__ int potrf_pivots8(double (&a)[8][8], double (&x)[8], 
 // for its four inverses; this takes 16.7k for both.
 // Returns the block's first non-positive pivot (zero pivot when !factor), or
 // -1; such a pivot is taken as 1.  Without factor, sM may be sL: the inverse
-// takes the block's place.
-template <int LD, int LDM>
+// takes the block's place.  !INV: no inverse, 1 / L(j, j) at sM[j] instead.
+template <int LD, int LDM, bool INV = true>
 __device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw, bool factor, int cols = 16) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, c8 = lane & 7;
   int first_bad = -1;
@@ -83,33 +83,41 @@ __device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw
       }
       __syncwarp();  // in place: every lane has read the block
     }
-    // column b0 + first of the inverse, right-looking: as soon as M(l, c) is
-    // known it is added into the partial sums of the later rows
-    const int first = h == 0 ? c8 : (lane & 15) - 8;
-    double m[8], t[8];
+    if (!INV) {
+      if (lane == 0) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) t[i] = first < 0 ? sTw[8 * c8 + i] : 0.0;
-#pragma unroll
-    for (int l = 0; l < 8; l++) {
-      m[l] = l == first ? r[l] : (l > first ? -r[l] * t[l] : 0.0);
-#pragma unroll
-      for (int i = l + 1; i < 8; i++) t[i] = fma(a[l][i], m[l], t[i]);
-    }
-    if (lane < (h == 0 ? 8 : 16)) {
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-        if (i >= first) sM[(b0 + first) * LDM + b0 + i] = m[i];
-    }
-    __syncwarp();
-    if (h == 0 && cols > 8) {
-      // what the first eight columns of the inverse start the second half
-      // with: L21 M11, column-major
-      double v[2] = {0.0, 0.0};
-#pragma unroll
-      for (int k = 0; k < 8; k += 4) dmma8(v, sL[(k + q) * LD + 8 + g], sM[g * LDM + k + q]);
-      sTw[16 * q + g] = v[0];
-      sTw[16 * q + 8 + g] = v[1];
+        for (int j = 0; j < 8; j++) sM[b0 + j] = r[j];
+      }
       __syncwarp();
+    } else {
+      // column b0 + first of the inverse, right-looking: as soon as M(l, c) is
+      // known it is added into the partial sums of the later rows
+      const int first = h == 0 ? c8 : (lane & 15) - 8;
+      double m[8], t[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) t[i] = first < 0 ? sTw[8 * c8 + i] : 0.0;
+#pragma unroll
+      for (int l = 0; l < 8; l++) {
+        m[l] = l == first ? r[l] : (l > first ? -r[l] * t[l] : 0.0);
+#pragma unroll
+        for (int i = l + 1; i < 8; i++) t[i] = fma(a[l][i], m[l], t[i]);
+      }
+      if (lane < (h == 0 ? 8 : 16)) {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          if (i >= first) sM[(b0 + first) * LDM + b0 + i] = m[i];
+      }
+      __syncwarp();
+      if (h == 0 && cols > 8) {
+        // what the first eight columns of the inverse start the second half
+        // with: L21 M11, column-major
+        double v[2] = {0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 8; k += 4) dmma8(v, sL[(k + q) * LD + 8 + g], sM[g * LDM + k + q]);
+        sTw[16 * q + g] = v[0];
+        sTw[16 * q + 8 + g] = v[1];
+        __syncwarp();
+      }
     }
     if (factor && h == 0) {
       // the second diagonal block: A(r, c) -= sum_k L(r, k) L(c, k), lower part
@@ -125,6 +133,6 @@ __device__ __forceinline__ int potrf_block16(double* sL, double* sM, double* sTw
       __syncwarp();
     }
   }
-  if (cols <= 8 && lane < 8) sM[(8 + lane) * LDM + 8 + lane] = 1.0;  // the second half is the identity, as L's is
+  if (INV && cols <= 8 && lane < 8) sM[(8 + lane) * LDM + 8 + lane] = 1.0;  // the second half is the identity, as L's is
   return first_bad;
 }

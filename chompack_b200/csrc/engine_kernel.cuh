@@ -1778,20 +1778,24 @@ static __device__ void run_asm(const RunArgs& ra, const Task& t, double* smem) {
 // separators from row and column NP on.
 //   1. F = the block's lower trapezoid, zero elsewhere;
 //   2. the children's update matrices added, last child first;
-//   3. the pivot columns eliminated in 16-column blocks as in the diagonal
-//      tile tasks (run_potrf), the separators as further rows below them,
-//      which leaves L11, L21 and the Schur complement F22 - L21 L21^T;
+//   3. the pivot columns eliminated in 16-column blocks, the separators as
+//      further rows below them, which leaves L11, L21 and the Schur
+//      complement F22 - L21 L21^T: a diagonal block by a warp
+//      (potrf_block16), the rows below it by substitution, a lane per row,
+//      the update of the rest by MMAs;
 //   4. the rows below replaced by W = L21 L11^{-1} (the reference's layout
 //      of the off-diagonal block): by 16-column blocks, last to first,
-//      W_J = (L21_J - sum_{K > J} W_K L(K, J)) Minv_JJ, a warp per 16 rows;
+//      W_J = (L21_J - sum_{K > J} W_K L(K, J)) L(J, J)^{-1}, the sum by MMAs
+//      and the rest by substitution, a warp per 16 rows;
 //   5. the block and the update matrix (operand c) written back.
 // A non-positive pivot records ctl[2] = j + 1 and continues with 1.
 // Bound by its chain of steps: with a barrier a pivot and scalar updates a
 // front of 2-D 30^2 (merged) took 34.2 us, in blocks 13.7.
+// (Substitution, not products with the inverses of the blocks: those leave a
+// residual that grows with the block's condition, 7e-15 at 4e3.)
 constexpr int FRONT_LD = TILE + 20;             // up to 80 rows; 4 mod 16
-constexpr int FRONT_DLD = 20;                   // the inverses of the diagonal blocks
-constexpr int FRONT_D = (TILE + 16) * FRONT_LD;
-static_assert(FRONT_D + TILE * FRONT_DLD + 64 + TILE / 2 <= ENGINE_SMEM_BASE_DOUBLES,
+constexpr int FRONT_D = (TILE + 16) * FRONT_LD; // 1 / L(j, j)
+static_assert(FRONT_D + TILE + TILE / 2 <= ENGINE_SMEM_BASE_DOUBLES,
               "small fronts exceed the engine's shared memory");
 
 // Up to this many pivots are eliminated one by one (a padded block of 16 costs
@@ -1844,17 +1848,70 @@ __device__ __forceinline__ void front_scalar(const RunArgs& ra, double* F, doubl
   __syncthreads();
 }
 
+// Rows [r0, r0 + 16) below the diagonal block in columns and rows j0 .. j0 + 16
+// of F, in place: x L(J, J)^T = A(r, J), lane mod 16 a row, rd = 1 / L(j, j).
+// The padding (columns from cols on, rows nn .. NP) stays zero whatever the
+// rows hold.
+__device__ __forceinline__ void front_panel_rows(double* F, const double* rd, int j0, int r0, int cols, int nn,
+                                                 int NP) {
+  constexpr int LD = FRONT_LD;
+  const int r = r0 + (threadIdx.x & 15);
+  double* const f = F + j0 * LD + r;
+  const double* const d = F + j0 * LD + j0;
+  double x[16];
+#pragma unroll
+  for (int c = 0; c < 16; c++) x[c] = f[c * LD];
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    x[j] *= rd[j];
+#pragma unroll
+    for (int c = (j + 1) & ~1; c < 16; c += 2) {
+      const double2 l = *reinterpret_cast<const double2*>(d + j * LD + c);
+      if (c > j) x[c] = fma(-x[j], l.x, x[c]);
+      x[c + 1] = fma(-x[j], l.y, x[c + 1]);
+    }
+  }
+  const bool row = r < nn || r >= NP;
+  __syncwarp();
+  if ((threadIdx.x & 16) == 0) {
+#pragma unroll
+    for (int c = 0; c < 16; c++) f[c * LD] = (row && c < cols) ? x[c] : 0.0;
+  }
+  __syncwarp();
+}
+
+// The same rows' x L(J, J) = B(r, J), columns last to first.
+__device__ __forceinline__ void front_solve_rows(double* F, const double* rd, int j0, int r0, int cols) {
+  constexpr int LD = FRONT_LD;
+  double* const f = F + j0 * LD + r0 + (threadIdx.x & 15);
+  const double* const d = F + j0 * LD + j0;
+  double x[16];
+#pragma unroll
+  for (int c = 0; c < 16; c++) x[c] = f[c * LD];
+#pragma unroll
+  for (int j = 15; j >= 0; j--) {
+    x[j] = j < cols ? x[j] * rd[j] : 0.0;
+#pragma unroll
+    for (int c = 0; c < j; c++) x[c] = fma(-x[j], d[c * LD + j], x[c]);
+  }
+  __syncwarp();
+  if ((threadIdx.x & 16) == 0) {
+#pragma unroll
+    for (int c = 0; c < 16; c++) f[c * LD] = x[c];
+  }
+  __syncwarp();
+}
+
 static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem) {
-  constexpr int LD = FRONT_LD, LDM = FRONT_DLD, NW = NTHREADS / 32;
+  constexpr int LD = FRONT_LD, NW = NTHREADS / 32;
   const FrontDesc f = ra.fronts[t.aux[0]];
   const int nn = f.nn, na = f.na, nj = f.nj;
   const bool blocked = nn > FRONT_SCALAR_NN;
   const int NJ = blocked ? (nn + 15) >> 4 : 0, NP = blocked ? 16 * NJ : nn, pad = NP - nn;
   const int NB = (NP + na + 15) >> 4, NF = blocked ? 16 * NB : nj;  // order of F
   double* F = smem;
-  double* D = smem + FRONT_D;         // block J's inverse at D + J * 16 * LDM
-  double* sT = D + TILE * LDM;
-  int* sr = reinterpret_cast<int*>(sT + 64);
+  double* rd = smem + FRONT_D;        // 1 / L(j, j)
+  int* sr = reinterpret_cast<int*>(rd + TILE);
   double* __restrict__ X = ra.bases[t.a.base] + t.a.off;
   double* __restrict__ U = ra.bases[t.c.base] + t.c.off;
   const int ldu = t.c.ld;
@@ -1881,8 +1938,6 @@ static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem)
         if (c < NF && r < NF) F[c * LD + r] = v[u][e];
       }
   }
-  if (blocked)
-    for (int i = tid; i < NP * LDM; i += NTHREADS) D[i] = 0.0;
   __syncthreads();
   // the children's update matrices, last child first: its relative indices
   // staged in shared memory, then the lower triangle of U_c flattened over
@@ -1916,7 +1971,7 @@ static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem)
     __syncthreads();
   }
   if (!blocked) {
-    front_scalar(ra, F, D, nn, nj);
+    front_scalar(ra, F, rd, nn, nj);
   }
   // step J: warp 0 the panel rows, the update and the factor of diagonal
   // block J, warps 1-3 the other panel rows of block J - 1 and the updates
@@ -1924,19 +1979,24 @@ static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem)
 #pragma unroll 1
   for (int J = 0; J < NJ; J++) {
     const int j0 = 16 * J, jp = j0 - 16;
-    const double* Mp = D + (J - 1) * 16 * LDM;
     if (warp == 0) {
       if (J > 0) {
-        potrf_panel_rows<LD, LDM>(F + jp * LD, Mp, j0);
+        front_panel_rows(F, rd + jp, jp, j0, 16, nn, NP);
         named_bar_arrive(1, NTHREADS);
         potrf_syrk_tile<LD>(F, jp, j0, j0);
         potrf_syrk_tile<LD>(F, jp, j0, j0 + 8);
         __syncwarp();
       }
-      const int bad = potrf_block16<LD, LDM>(F + j0 * LD + j0, D + J * 16 * LDM, sT, true, min(16, nn - j0));
-      if (lane == 0 && bad >= 0) atomicCAS(&ra.ctl[2], 0, j0 + bad + 1);
+      const int cols = min(16, nn - j0);
+      const int bad = potrf_block16<LD, LD, false>(F + j0 * LD + j0, rd + j0, nullptr, true, cols);
+      if (lane == 0 && bad >= 0 && bad < cols) atomicCAS(&ra.ctl[2], 0, j0 + bad + 1);
+      if (cols < 16) {  // the padded rows of the block, whatever the pivots left there
+        __syncwarp();
+        for (int i = lane; i < 256; i += 32)
+          if ((i >> 4) < cols && (i & 15) >= cols) F[(j0 + (i >> 4)) * LD + j0 + (i & 15)] = 0.0;
+      }
     } else if (J > 0) {
-      for (int rb = J + warp; rb < NB; rb += NW - 1) potrf_panel_rows<LD, LDM>(F + jp * LD, Mp, 16 * rb);
+      for (int rb = J + warp; rb < NB; rb += NW - 1) front_panel_rows(F, rd + jp, jp, 16 * rb, 16, nn, NP);
       named_bar_sync(1, NTHREADS);
       int at = 0;
       for (int I = J + 1; I < NB; I++)
@@ -1947,7 +2007,7 @@ static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem)
   }
   if (blocked && na > 0) {
     const int jp = NP - 16;
-    for (int rb = NJ + warp; rb < NB; rb += NW) potrf_panel_rows<LD, LDM>(F + jp * LD, D + (NJ - 1) * 16 * LDM, 16 * rb);
+    for (int rb = NJ + warp; rb < NB; rb += NW) front_panel_rows(F, rd + jp, jp, 16 * rb, nn - jp, nn, NP);
     __syncthreads();
     int at = 0;
     for (int I = NJ; I < NB; I++)
@@ -1960,8 +2020,8 @@ static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem)
 #pragma unroll 1
       for (int J = NJ - 1; J >= 0; J--) {
         double* const d = F + (16 * J + 2 * q) * LD + r0 + g;
-        double acc[2][4];
         if (J < NJ - 1) {
+          double acc[2][4];
 #pragma unroll
           for (int e = 0; e < 2; e++) {
 #pragma unroll
@@ -1976,18 +2036,7 @@ static __device__ void run_front(const RunArgs& ra, const Task& t, double* smem)
             for (int h = 0; h < 4; h++) d[(8 * e + (h & 1)) * LD + (h & 2) * 4] = acc[e][h];
           __syncwarp();
         }
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-#pragma unroll
-          for (int h = 0; h < 4; h++) acc[e][h] = 0.0;
-          warp_mma_16x8<false>(acc[e], F + 16 * J * LD + r0, LD, D + J * 16 * LDM + 8 * e * LDM, 1, LDM, 16);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int e = 0; e < 2; e++)
-#pragma unroll
-          for (int h = 0; h < 4; h++) d[(8 * e + (h & 1)) * LD + (h & 2) * 4] = acc[e][h];
-        __syncwarp();
+        front_solve_rows(F, rd + 16 * J, 16 * J, r0, nn - 16 * J);
       }
     }
     __syncthreads();
@@ -3156,7 +3205,7 @@ static_assert(8 * SUB_NJ * SUB_LD <= ENGINE_SMEM_BASE_DOUBLES, "bundle fronts ex
 template <int BUILD>
 __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
   constexpr bool TC = BUILD == EB_TCGEN05;
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   __shared__ int s_task;
   __shared__ int s_abort;
   __shared__ int s_next;      // dynamic: the waiter this CTA released and runs next, or -1

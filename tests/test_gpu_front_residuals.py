@@ -1,0 +1,59 @@
+"""Backward errors of cholesky on small fronts whose pivot block is
+ill-conditioned: the factor and the rows below it, componentwise, for fronts
+of their own task (bundles off) and for bundles."""
+import numpy as np
+import pytest
+import torch
+
+import chompack_b200 as cp
+from chompack_b200 import grids
+
+pytestmark = pytest.mark.gpu
+
+U = 2.0 ** -53
+EXTRA = 3
+
+
+def kahan(n, rng, angle):
+    c, s = np.cos(angle), np.sin(angle)
+    return (np.eye(n) - c * np.tril(np.ones((n, n)), -1)) * s ** (np.arange(n) % 16) * (1 + 0.1 * rng.random((n, n)))
+
+
+def front(nn, na, seed):
+    """Block values of a front of nn columns and na rows below them, under a
+    root of na + EXTRA columns; A11 = L11 L11^T with L11 ill-conditioned."""
+    rng = np.random.default_rng(seed)
+    L = kahan(nn, rng, 1.0 if nn <= 24 else 1.25).astype(np.longdouble)
+    W = rng.standard_normal((na, nn)).astype(np.longdouble)
+    A11 = (L @ L.T).astype(np.float64)
+    A21 = (W @ L @ L.T).astype(np.float64)
+    nr = na + EXTRA
+    R = np.tril(rng.standard_normal((nr, nr))) + 3 * np.eye(nr)
+    A22 = R @ R.T
+    A22[:na, :na] += ((W @ L) @ (W @ L).T).astype(np.float64)
+    return A11, A21, A22
+
+
+@pytest.mark.parametrize("bundles", [0, 1])
+@pytest.mark.parametrize("nn,na", [(3, 20), (5, 11), (9, 20), (16, 16), (16, 40), (24, 33), (33, 31), (47, 17)])
+def test_backward_error(nn, na, bundles):
+    if bundles and nn + na > 32:
+        pytest.skip("bundles hold fronts of at most 32 rows")
+    n = nn + na + EXTRA
+    r, c = np.tril_indices(n, -1)
+    keep = (c >= nn) | (r < nn + na)
+    s = cp.symbolic(grids.spd_from_lower_pattern(n, r[keep], c[keep], 0))
+    assert [int(x) for x in np.diff(s.snptr)] == [nn, na + EXTRA]
+    s.plan().set_option("subtrees", bundles)
+    A11, A21, A22 = front(nn, na, 10 * nn + na)
+    x = np.concatenate([np.concatenate([np.tril(A11), A21]).ravel(order="F"), np.tril(A22).ravel(order="F")])
+    X = cp.cspmatrix(s, blkval=torch.from_numpy(x).cuda())
+    cp.cholesky(X)
+    got = X.blkval.cpu().numpy()[:(nn + na) * nn].reshape(nn, nn + na).T.astype(np.longdouble)
+    L, W = np.tril(got[:nn]), got[nn:]
+    # |A11 - L L^T| <= gamma_(nn + 1) |L| |L^T|, and a few roundings for the
+    # reciprocals; W solves X L^T = A21, then W L = X, each within gamma_nn
+    g = (nn + 4) * U
+    aL = np.abs(L)
+    assert np.all(np.abs(A11 - L @ L.T) <= g * (aL @ aL.T))
+    assert np.all(np.abs(A21 - W @ (L @ L.T)) <= 2.1 * g * (np.abs(W) @ (aL @ aL.T)))
