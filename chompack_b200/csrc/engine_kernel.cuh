@@ -3053,23 +3053,19 @@ static __device__ void chol_front_warp(const RunArgs& ra, int k, double* F, int 
     __syncwarp();
   }
   // partial Cholesky of the nn pivot columns; the trailing block becomes U_k
-  // (1 / L(j, j) is kept behind row j)
   int first_bad = -1;
   for (int j = 0; j < nn; j++) {
     const double d = F[j * SUB_LD + j];
     const bool bad = !(d > 0.0);
     if (bad && first_bad < 0) first_bad = j;
-    const double x = bad ? 1.0 : d, rs = rsqrt(x);
+    const double lj = sqrt(bad ? 1.0 : d), rl = 1.0 / lj;
     double a = 0.0;
     if (lane > j && lane < nj) {
-      a = row[j] * rs;
+      a = row[j] * rl;
       row[j] = a;
     }
     __syncwarp();
-    if (lane == j) {
-      row[j] = x * rs;
-      row[SUB_NJ] = rs;
-    }
+    if (lane == j) row[j] = lj;
     for (int c0 = j + 1; c0 < nj; c0 += SUB_E) {
       double u[SUB_E], w[SUB_E];
 #pragma unroll
@@ -3090,7 +3086,7 @@ static __device__ void chol_front_warp(const RunArgs& ra, int k, double* F, int 
     for (int j = nn - 1; j >= 0; j--) {
       double v = row[j];
       for (int l2 = j + 1; l2 < nn; l2++) v = fma(-row[l2], F[l2 * SUB_LD + j], v);
-      row[j] = v * F[j * SUB_LD + SUB_NJ];
+      row[j] = v / F[j * SUB_LD + j];
     }
   __syncwarp();
   for (int c = 0; c < nn; c++)

@@ -1,6 +1,7 @@
 """Backward errors of cholesky on small fronts whose pivot block is
 ill-conditioned: the factor and the rows below it, componentwise, for fronts
-of their own task (bundles off) and for bundles."""
+of their own task (bundles off) and for bundles; the rounding and the range of
+a bundle's pivots."""
 import numpy as np
 import pytest
 import torch
@@ -57,3 +58,35 @@ def test_backward_error(nn, na, bundles):
     aL = np.abs(L)
     assert np.all(np.abs(A11 - L @ L.T) <= g * (aL @ aL.T))
     assert np.all(np.abs(A21 - W @ (L @ L.T)) <= 2.1 * g * (np.abs(W) @ (aL @ aL.T)))
+
+
+def test_bundle_pivots():
+    # leaves of one column under a root of four (the last leaf is in the root)
+    m, nr = 301, 4
+    r = np.concatenate([np.tile(np.arange(m, m + nr), m), m + np.tril_indices(nr, -1)[0]])
+    c = np.concatenate([np.repeat(np.arange(m), nr), m + np.tril_indices(nr, -1)[1]])
+    s = cp.symbolic(grids.spd_from_lower_pattern(m + nr, r, c, 0))
+    nn = np.diff(s.snptr)
+    assert s.Nsn == m and np.count_nonzero(nn == 1) == m - 1
+    rng = np.random.default_rng(1)
+    x = np.zeros(int(s.blkptr[-1]))
+    at = np.array([int(s.blkptr[k]) for k in range(m) if nn[k] == 1])
+    x[at] = rng.uniform(1.0, 4.0, m - 1)
+    x[at[:, None] + np.arange(1, nr + 1)] = rng.standard_normal((m - 1, nr))
+    k = int(np.argmax(nn))
+    root = slice(int(s.blkptr[k]), int(s.blkptr[k + 1]))
+    x[root][::nr + 2] = 10.0 * m
+
+    def factor(v):
+        X = cp.cspmatrix(s, blkval=torch.from_numpy(v.copy()).cuda())
+        cp.cholesky(X)
+        return X.blkval.cpu().numpy()
+
+    L = factor(x)
+    assert np.array_equal(L[at], np.sqrt(x[at]))
+    # an infinite pivot: its column vanishes, the other leaves stay as they are
+    x[at[7]] = np.inf
+    Li = factor(x)
+    assert Li[at[7]] == np.inf and not np.any(Li[at[7] + 1:at[7] + 1 + nr])
+    other = np.delete(at, 7)[:, None] + np.arange(nr + 1)
+    assert np.array_equal(Li[other], L[other]) and np.all(np.isfinite(Li[root]))
