@@ -2085,6 +2085,34 @@ __device__ __forceinline__ void warp_mma_any(double (&acc)[4], const double* pa,
 constexpr int PF_LD = TILE + 4;
 static_assert(2 * TILE * PF_LD + 4 * 64 + TILE / 2 + 8 <= ENGINE_SMEM_BASE_DOUBLES,
               "small fronts exceed the engine's shared memory");
+
+// M = L11^{-1} in place in G, column by column from the last (as LAPACK's
+// unblocked triangular inverse), and Y11 = M^T M into F, by scalar dots that
+// touch no zero of the triangles: for an L11 with infinities or NaN, which the
+// zeros in the MMAs' tiles would spread to entries that do not depend on them.
+__device__ __forceinline__ void pfront_scalar(double* G, double* F, int nn) {
+  constexpr int LD = PF_LD, NW = NTHREADS / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int j = nn - 1; j >= 0; j--) {
+    const double d = G[j * LD + j], ajj = 1.0 / (d == 0.0 ? 1.0 : d);
+    const int i = j + 1 + tid;
+    double v = 0.0;
+    if (i < nn)
+      for (int l = j + 1; l <= i; l++) v = fma(G[l * LD + i], G[j * LD + l], v);
+    __syncthreads();
+    if (i < nn) G[j * LD + i] = -ajj * v;
+    if (tid == 0) G[j * LD + j] = ajj;
+    __syncthreads();
+  }
+  for (int j = warp; j < nn; j += NW)
+    for (int i = j + lane; i < nn; i += 32) {
+      double v = 0.0;
+      for (int l = i; l < nn; l++) v = fma(G[i * LD + l], G[j * LD + l], v);
+      F[j * LD + i] = v;
+    }
+  __syncthreads();
+}
+
 static __device__ void run_pfront(const RunArgs& ra, const Task& t, double* smem) {
   constexpr int LD = PF_LD, NW = NTHREADS / 32;
   const FrontDesc f = ra.fronts[t.aux[0]];
@@ -2100,6 +2128,7 @@ static __device__ void run_pfront(const RunArgs& ra, const Task& t, double* smem
   const int ldv = t.c.ld;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   if (tid == 0) *s_bad = -1;
+  bool finite = true;
   // (four columns' loads at a time: a load is not moved above a store to
   // shared memory)
   for (int c4 = warp; c4 < NP; c4 += 4 * NW) {
@@ -2118,6 +2147,7 @@ static __device__ void run_pfront(const RunArgs& ra, const Task& t, double* smem
         const int c = c4 + u * NW, r = lane + 32 * e;
         if (r < NP) G[c * LD + r] = (c < nn && r < nn) ? (r >= c ? v[u][e] : 0.0) : (r == c ? 1.0 : 0.0);
         if (c < nn && r >= nn && r < nj) F[c * LD + r] = v[u][e];
+        finite = finite && (r < c || r >= nn || isfinite(v[u][e]));
       }
   }
   for (int c4 = warp; c4 < na; c4 += 4 * NW) {
@@ -2140,53 +2170,58 @@ static __device__ void run_pfront(const RunArgs& ra, const Task& t, double* smem
         }
       }
   }
-  __syncthreads();
+  finite = __syncthreads_and(finite);
   if (tid < nn && G[tid * LD + tid] == 0.0) atomicMax(s_bad, tid);
   __syncthreads();
   if (tid == 0 && *s_bad >= 0) atomicCAS(&ra.ctl[2], 0, *s_bad + 1);
-  // M in place of L11
-  if (warp < NJ) {
-    double* d = G + 16 * warp * LD + 16 * warp;
-    potrf_block16<LD, LD>(d, d, sT + 64 * warp, false, min(16, nn - 16 * warp));
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (int I = 1; I < NJ; I++) {
-    // L(I, :I) M(:I, tile) of at most two tiles a warp, then in their place
-    double ac[2][4];
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const int tj = warp + NW * e;
-      ac[e][0] = ac[e][1] = ac[e][2] = ac[e][3] = 0.0;
-      if (tj < 2 * I) warp_mma_any<false>(ac[e], G + 16 * I, 1, LD, G + 8 * tj * LD, 1, LD, 16 * (tj / 2), 16 * I);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const int tj = warp + NW * e;
-      if (tj >= 2 * I) continue;
-      double* d = G + (8 * tj + 2 * q) * LD + 16 * I + g;
-#pragma unroll
-      for (int h = 0; h < 4; h++) d[(h & 1) * LD + (h & 2) * 4] = ac[e][h];
-      __syncwarp();
-      potrf_inv_finish(G, I, tj);
-    }
-    __syncthreads();
-  }
-  // Y11 = M^T M: tiles of 16 x 8 on and below the diagonal
   int at = 0;
-  for (int I = 0; I < NJ; I++)
-    for (int c0 = 0; c0 < min(16 * I + 16, nn); c0 += 8) {
-      if (at++ % NW != warp) continue;
-      double y[4] = {0.0, 0.0, 0.0, 0.0};
-      warp_mma_any<false>(y, G + 16 * I * LD, LD, 1, G + c0 * LD, 1, LD, 16 * I, NP);
-#pragma unroll
-      for (int h = 0; h < 4; h++) {
-        const int r = 16 * I + g + (h & 2) * 4, c = c0 + 2 * q + (h & 1);
-        if (r < nn && c <= r) F[c * LD + r] = y[h];
-      }
+  if (!finite) {
+    pfront_scalar(G, F, nn);
+  } else {
+    // M in place of L11
+    if (warp < NJ) {
+      double* d = G + 16 * warp * LD + 16 * warp;
+      potrf_block16<LD, LD>(d, d, sT + 64 * warp, false, min(16, nn - 16 * warp));
     }
-  __syncthreads();
+    __syncthreads();
+#pragma unroll 1
+    for (int I = 1; I < NJ; I++) {
+      // L(I, :I) M(:I, tile) of at most two tiles a warp, then in their place
+      double ac[2][4];
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int tj = warp + NW * e;
+        ac[e][0] = ac[e][1] = ac[e][2] = ac[e][3] = 0.0;
+        if (tj < 2 * I) warp_mma_any<false>(ac[e], G + 16 * I, 1, LD, G + 8 * tj * LD, 1, LD, 16 * (tj / 2), 16 * I);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int tj = warp + NW * e;
+        if (tj >= 2 * I) continue;
+        double* d = G + (8 * tj + 2 * q) * LD + 16 * I + g;
+#pragma unroll
+        for (int h = 0; h < 4; h++) d[(h & 1) * LD + (h & 2) * 4] = ac[e][h];
+        __syncwarp();
+        potrf_inv_finish(G, I, tj);
+      }
+      __syncthreads();
+    }
+    // Y11 = M^T M: tiles of 16 x 8 on and below the diagonal
+    at = 0;
+    for (int I = 0; I < NJ; I++)
+      for (int c0 = 0; c0 < min(16 * I + 16, nn); c0 += 8) {
+        if (at++ % NW != warp) continue;
+        double y[4] = {0.0, 0.0, 0.0, 0.0};
+        warp_mma_any<false>(y, G + 16 * I * LD, LD, 1, G + c0 * LD, 1, LD, 16 * I, NP);
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+          const int r = 16 * I + g + (h & 2) * 4, c = c0 + 2 * q + (h & 1);
+          if (r < nn && c <= r) F[c * LD + r] = y[h];
+        }
+      }
+    __syncthreads();
+  }
   if (na > 0) {
     // S21 = -V W into G
     at = 0;

@@ -1,7 +1,7 @@
 """Backward errors of cholesky on small fronts whose pivot block is
 ill-conditioned: the factor and the rows below it, componentwise, for fronts
 of their own task (bundles off) and for bundles; the rounding and the range of
-a bundle's pivots."""
+a bundle's pivots; a value that is not finite in projected_inverse."""
 import numpy as np
 import pytest
 import torch
@@ -90,3 +90,22 @@ def test_bundle_pivots():
     assert Li[at[7]] == np.inf and not np.any(Li[at[7] + 1:at[7] + 1 + nr])
     other = np.delete(at, 7)[:, None] + np.arange(nr + 1)
     assert np.array_equal(Li[other], L[other]) and np.all(np.isfinite(Li[root]))
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("n,row,col", [(20, 17, 3), (40, 20, 3), (40, 39, 17), (64, 50, 30), (33, 32, 0)])
+def test_non_finite_entry_stays_in_its_columns(n, row, col, value):
+    # one front; Y(i, j) depends on L(row, col) only where min(i, j) <= col
+    A = grids.random_lower(n, 1.0, seed=n)
+    s = cp.symbolic(A)
+    assert s.Nsn == 1
+    s.plan().set_option("subtrees", 0)
+    M = (cp.cspmatrix(s, device="cpu") + A).blkval.numpy().reshape(n, n, order="F")
+    L = np.linalg.cholesky(np.tril(M) + np.tril(M, -1).T)
+    T = np.linalg.inv(L[col + 1:, col + 1:])
+    L[row, col] = value
+    X = cp.cspmatrix(s, blkval=torch.from_numpy(L.ravel(order="F").copy()).cuda(), factor=True)
+    cp.projected_inverse(X)
+    Y = X.blkval.cpu().numpy().reshape(n, n, order="F")[col + 1:, col + 1:]
+    want = np.tril(T.T @ T)
+    assert np.all(np.abs(np.tril(Y) - want) <= 1e-13 * np.abs(want).max())
