@@ -1047,7 +1047,7 @@ __device__ __forceinline__ bool is_narrow(const Task& t) {
   return BUILD == EB_SOLVE && t.op == T_GEMM && t.aux[0] == GEMM_NARROW;
 }
 
-static __device__ void run_trsv(const RunArgs& ra, const Task& t, double* smem, int& claim) {
+static __device__ void run_trsv(const RunArgs& ra, const Task& t, double* smem, int ti, int& claim) {
   __shared__ int s_trsv_abort;
   constexpr int LA = TRSV_LA, LB = TRSV_LB;
   double* sA = smem;
@@ -1092,6 +1092,8 @@ static __device__ void run_trsv(const RunArgs& ra, const Task& t, double* smem, 
       }
     }
     s_trsv_abort = abort;
+    // a narrow product's dependencies are met now, not when it was claimed
+    if (ra.trace && t.op == T_GEMM && !ra.dynamic) ra.trace[4 * (int64_t)ti + 1] = global_ns();
   }
   __syncthreads();
   if (s_trsv_abort) {
@@ -3389,7 +3391,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
         else if (threadIdx.x == 0) atomicCAS(&ra.ctl[1], 0, DE_BAD_TASK);
         break;
       case T_TRSV:
-        if (BUILD == EB_SOLVE) run_trsv(ra, t, smem, claim);
+        if (BUILD == EB_SOLVE) run_trsv(ra, t, smem, ti, claim);
         else if (threadIdx.x == 0) atomicCAS(&ra.ctl[1], 0, DE_BAD_TASK);
         break;
       case T_QL:

@@ -347,8 +347,10 @@ int chb_dot_batch(chb_plan* plan, const double* x, const double* y, double* resu
 
 /* Profiling: when `buffer` (device memory, 32 bytes per task) is set, the
  * next sweeps whose task count fits `capacity_tasks` record per task the
- * global-timer ns at claim, start (dependencies met) and end, and the SM id
- * | task kind << 32.  Pass NULL to switch tracing off. */
+ * global-timer ns at claim, start (dependencies met; those it starts with
+ * for a task that waits once more inside: a step of a solve, a fused
+ * diagonal task) and end, and the SM id | task kind << 32.  Pass NULL to
+ * switch tracing off. */
 int chb_set_trace(chb_plan* plan, void* buffer, int64_t capacity_tasks);
 
 /* Task scheduling of the plan's sweeps: 0 dynamic (a finished task releases
