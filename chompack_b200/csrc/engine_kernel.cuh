@@ -1882,20 +1882,26 @@ __device__ __forceinline__ void front_panel_rows(double* F, const double* rd, in
   __syncwarp();
 }
 
-// The same rows' x L(J, J) = B(r, J), columns last to first.
-__device__ __forceinline__ void front_solve_rows(double* F, const double* rd, int j0, int r0, int cols) {
-  constexpr int LD = FRONT_LD;
-  double* const f = F + j0 * LD + r0 + (threadIdx.x & 15);
-  const double* const d = F + j0 * LD + j0;
-  double x[16];
-#pragma unroll
-  for (int c = 0; c < 16; c++) x[c] = f[c * LD];
+// x := x L^{-1} for a row x of 16 columns, last to first, L(j, c) = d[c * LD + j],
+// rd = 1 / L(j, j); the columns from cols on are zero.
+template <int LD>
+__device__ __forceinline__ void solve_row16(double (&x)[16], const double* d, const double* rd, int cols) {
 #pragma unroll
   for (int j = 15; j >= 0; j--) {
     x[j] = j < cols ? x[j] * rd[j] : 0.0;
 #pragma unroll
     for (int c = 0; c < j; c++) x[c] = fma(-x[j], d[c * LD + j], x[c]);
   }
+}
+
+// The same rows' x L(J, J) = B(r, J).
+__device__ __forceinline__ void front_solve_rows(double* F, const double* rd, int j0, int r0, int cols) {
+  constexpr int LD = FRONT_LD;
+  double* const f = F + j0 * LD + r0 + (threadIdx.x & 15);
+  double x[16];
+#pragma unroll
+  for (int c = 0; c < 16; c++) x[c] = f[c * LD];
+  solve_row16<LD>(x, F + j0 * LD + j0, rd, cols);
   __syncwarp();
   if ((threadIdx.x & 16) == 0) {
 #pragma unroll
@@ -2075,8 +2081,11 @@ __device__ __forceinline__ void warp_mma_any(double (&acc)[4], const double* pa,
 // A whole small projected-inverse front (T_PFRONT, nj <= TILE;
 // projected_inverse.c:33-73 for one node) in shared memory: G holds L11,
 // padded with an identity to a multiple of 16 columns, then M = L11^{-1} in
-// its place (diagonal 16 x 16 blocks by a warp each, then block row by block
-// row), then S21; F holds the front: W and V_k (operand c, both triangles)
+// its place, then S21; M by block columns, last to first,
+//   M(I, J) L(J, J) = -sum_{J < K <= I} M(I, K) L(K, J)   (the identity for I = J),
+// the sum by MMAs and the rest by substitution, a lane per row (block rows
+// times the diagonal blocks' inverses lost up to a third more digits on
+// ill-conditioned fronts); F holds the front: W and V_k (operand c, both triangles)
 // first, then [Y11; S21 | V_k].
 //   Y11 = M^T M;  S21 = -V_k W;  Y11 -= S21^T W   (FP64 MMAs);
 //   U_c = F(r_c, r_c) for every child c (lower parts);
@@ -2085,7 +2094,7 @@ __device__ __forceinline__ void warp_mma_any(double (&acc)[4], const double* pa,
 // With scalar dots, two barriers a column of M, a front of 2-D 30^2 (merged)
 // took 24.1 us, now 12.0.
 constexpr int PF_LD = TILE + 4;
-static_assert(2 * TILE * PF_LD + 4 * 64 + TILE / 2 + 8 <= ENGINE_SMEM_BASE_DOUBLES,
+static_assert(2 * TILE * PF_LD + TILE + TILE / 2 + 8 <= ENGINE_SMEM_BASE_DOUBLES,
               "small fronts exceed the engine's shared memory");
 
 // M = L11^{-1} in place in G, column by column from the last (as LAPACK's
@@ -2122,8 +2131,8 @@ static __device__ void run_pfront(const RunArgs& ra, const Task& t, double* smem
   const int NJ = (nn + 15) >> 4, NP = 16 * NJ;
   double* F = smem;
   double* G = smem + TILE * LD;
-  double* sT = G + TILE * LD;
-  int* sr = reinterpret_cast<int*>(sT + NW * 64);
+  double* rd = G + TILE * LD;         // 1 / L(j, j)
+  int* sr = reinterpret_cast<int*>(rd + TILE);
   int* s_bad = sr + TILE;
   double* __restrict__ X = ra.bases[t.a.base] + t.a.off;
   const double* __restrict__ V = ra.bases[t.c.base] + t.c.off;
@@ -2173,39 +2182,50 @@ static __device__ void run_pfront(const RunArgs& ra, const Task& t, double* smem
       }
   }
   finite = __syncthreads_and(finite);
-  if (tid < nn && G[tid * LD + tid] == 0.0) atomicMax(s_bad, tid);
+  if (tid < NP) {
+    const double d = G[tid * LD + tid];
+    if (d == 0.0) atomicMax(s_bad, tid);
+    rd[tid] = 1.0 / (d == 0.0 ? 1.0 : d);
+  }
   __syncthreads();
   if (tid == 0 && *s_bad >= 0) atomicCAS(&ra.ctl[2], 0, *s_bad + 1);
   int at = 0;
   if (!finite) {
     pfront_scalar(G, F, nn);
   } else {
-    // M in place of L11
-    if (warp < NJ) {
-      double* d = G + 16 * warp * LD + 16 * warp;
-      potrf_block16<LD, LD>(d, d, sT + 64 * warp, false, min(16, nn - 16 * warp));
-    }
-    __syncthreads();
+    // M in place of L11: block row J + warp of block column J (F's rows < nn
+    // are free and take the sums to their rows' lanes)
 #pragma unroll 1
-    for (int I = 1; I < NJ; I++) {
-      // L(I, :I) M(:I, tile) of at most two tiles a warp, then in their place
-      double ac[2][4];
+    for (int J = NJ - 1; J >= 0; J--) {
+      const int I = J + warp, r = 16 * I + (lane & 15);
+      double* const gj = G + 16 * J * LD;
+      double x[16];
+      if (I < NJ) {
+        if (warp == 0) {
 #pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int tj = warp + NW * e;
-        ac[e][0] = ac[e][1] = ac[e][2] = ac[e][3] = 0.0;
-        if (tj < 2 * I) warp_mma_any<false>(ac[e], G + 16 * I, 1, LD, G + 8 * tj * LD, 1, LD, 16 * (tj / 2), 16 * I);
+          for (int c = 0; c < 16; c++) x[c] = (lane & 15) == c ? 1.0 : 0.0;
+        } else {
+          double* const fj = F + 16 * J * LD;
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            double y[4] = {0.0, 0.0, 0.0, 0.0};
+            warp_mma_any<true>(y, G + 16 * I, 1, LD, gj + 8 * e * LD, 1, LD, 16 * (J + 1), 16 * (I + 1));
+#pragma unroll
+            for (int h = 0; h < 4; h++) {
+              const int row = 16 * I + g + (h & 2) * 4;
+              if (row < nn) fj[(8 * e + 2 * q + (h & 1)) * LD + row] = y[h];
+            }
+          }
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < 16; c++) x[c] = r < nn ? fj[c * LD + r] : 0.0;
+        }
+        solve_row16<LD>(x, gj + 16 * J, rd + 16 * J, 16);
       }
       __syncthreads();
+      if (I < NJ && lane < 16) {
 #pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int tj = warp + NW * e;
-        if (tj >= 2 * I) continue;
-        double* d = G + (8 * tj + 2 * q) * LD + 16 * I + g;
-#pragma unroll
-        for (int h = 0; h < 4; h++) d[(h & 1) * LD + (h & 2) * 4] = ac[e][h];
-        __syncwarp();
-        potrf_inv_finish(G, I, tj);
+        for (int c = 0; c < 16; c++) gj[c * LD + r] = x[c];
       }
       __syncthreads();
     }
@@ -3238,6 +3258,7 @@ static_assert(8 * SUB_NJ * SUB_LD <= ENGINE_SMEM_BASE_DOUBLES, "bundle fronts ex
 template <int BUILD>
 __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
   constexpr bool TC = BUILD == EB_TCGEN05;
+  constexpr bool FRONTS = BUILD == EB_BASE || TC;  // small fronts and bundles (cholesky, projected_inverse)
   extern __shared__ __align__(16) double smem[];
   __shared__ int s_task;
   __shared__ int s_abort;
@@ -3380,10 +3401,19 @@ __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
       case T_MROW: run_mrow(ra, t, sm); break;
       case T_POTRF: run_potrf(ra, t, smem, ti); break;
       case T_ASM: run_asm(ra, t, smem); break;
-      case T_FRONT: run_front(ra, t, smem); break;
-      case T_PFRONT: run_pfront(ra, t, smem); break;
+      case T_FRONT:
+        if (FRONTS) run_front(ra, t, smem);
+        else if (threadIdx.x == 0) atomicCAS(&ra.ctl[1], 0, DE_BAD_TASK);
+        break;
+      case T_PFRONT:
+        if (FRONTS) run_pfront(ra, t, smem);
+        else if (threadIdx.x == 0) atomicCAS(&ra.ctl[1], 0, DE_BAD_TASK);
+        break;
       case T_SUBTREE:
-      case T_PSUBTREE: run_subtrees(ra, t, smem); break;
+      case T_PSUBTREE:
+        if (FRONTS) run_subtrees(ra, t, smem);
+        else if (threadIdx.x == 0) atomicCAS(&ra.ctl[1], 0, DE_BAD_TASK);
+        break;
       case T_EXTRACT: run_extract(ra, t, smem); break;
       case T_COPY: run_copy(ra, t); break;
       case T_VEC:

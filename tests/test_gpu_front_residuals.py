@@ -109,3 +109,47 @@ def test_non_finite_entry_stays_in_its_columns(n, row, col, value):
     Y = X.blkval.cpu().numpy().reshape(n, n, order="F")[col + 1:, col + 1:]
     want = np.tril(T.T @ T)
     assert np.all(np.abs(np.tril(Y) - want) <= 1e-13 * np.abs(want).max())
+
+
+def fma(a, b, c):
+    return (np.asarray(a, np.longdouble) * b + c).astype(np.float64)
+
+
+def scalar_inverse(L):
+    """(L L^T)^{-1} as an unblocked inverse from the last column to the first
+    and sequential dots give it in double precision."""
+    n = len(L)
+    M, Y = L.copy(), np.zeros((n, n))
+    for j in range(n - 1, -1, -1):
+        a, t = 1.0 / M[j, j], np.zeros(n)
+        for k in range(j + 1, n):
+            t[k:] = fma(M[k:, k], M[k, j], t[k:])
+        M[j + 1:, j], M[j, j] = -a * t[j + 1:], a
+    for k in range(n):
+        Y = fma(M[k][:, None], M[k][None, :], Y)
+    return Y
+
+
+@pytest.mark.parametrize("n,decades", [(40, 6), (40, 10), (64, 10)])
+def test_inverse_is_as_exact_as_a_scalar_one(n, decades):
+    # 40 rotated spectra, one blocked front each; the two errors are those of
+    # two rounding sequences of one size, so their mean log ratio is within
+    # three standard errors of zero
+    s = cp.symbolic(grids.random_lower(n, 1.0, seed=n))
+    s.plan().set_option("subtrees", 0)
+    here, scalar = [], []
+    for seed in range(40):
+        Q = np.linalg.qr(np.random.default_rng(seed).standard_normal((n, n)))[0]
+        A = (Q * 10.0 ** np.linspace(0, -decades, n)) @ Q.T
+        L = np.linalg.cholesky((A + A.T) / 2)
+        T = np.eye(n, dtype=np.longdouble)
+        for i in range(n):
+            T[i] = (T[i] - L[i, :i] @ T[:i]) / L[i, i]
+        want = np.tril(T.T @ T)
+        X = cp.cspmatrix(s, blkval=torch.from_numpy(L.ravel(order="F").copy()).cuda(), factor=True)
+        cp.projected_inverse(X)
+        for e, Y in ((here, X.blkval.cpu().numpy().reshape(n, n, order="F")), (scalar, scalar_inverse(L))):
+            d = np.tril(Y) - want
+            e.append(float(np.sqrt(np.sum(d * d) / np.sum(want * want))))
+    ratio = np.log(np.array(here) / np.array(scalar))
+    assert ratio.mean() <= 3.0 * ratio.std(ddof=1) / np.sqrt(len(ratio)), (ratio.mean(), ratio.std())
