@@ -2259,22 +2259,18 @@ static __device__ void run_pfront(const RunArgs& ra, const Task& t, double* smem
         }
       }
     __syncthreads();
-    // Y11 -= S21^T W
+    // Y11 -= S21^T W (summed on its own: added one by one to the larger Y11
+    // the products would be rounded to its size each)
     at = 0;
     for (int I = 0; I < NJ; I++)
       for (int c0 = 0; c0 < min(16 * I + 16, nn); c0 += 8) {
         if (at++ % NW != warp) continue;
-        double y[4];
+        double y[4] = {0.0, 0.0, 0.0, 0.0};
+        warp_mma_any<false>(y, G + 16 * I * LD, LD, 1, F + c0 * LD + nn, 1, LD, 0, na);
 #pragma unroll
         for (int h = 0; h < 4; h++) {
           const int r = 16 * I + g + (h & 2) * 4, c = c0 + 2 * q + (h & 1);
-          y[h] = (r < nn && c <= r) ? F[c * LD + r] : 0.0;
-        }
-        warp_mma_any<true>(y, G + 16 * I * LD, LD, 1, F + c0 * LD + nn, 1, LD, 0, na);
-#pragma unroll
-        for (int h = 0; h < 4; h++) {
-          const int r = 16 * I + g + (h & 2) * 4, c = c0 + 2 * q + (h & 1);
-          if (r < nn && c <= r) F[c * LD + r] = y[h];
+          if (r < nn && c <= r) F[c * LD + r] -= y[h];
         }
       }
     __syncthreads();

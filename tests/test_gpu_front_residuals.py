@@ -153,3 +153,39 @@ def test_inverse_is_as_exact_as_a_scalar_one(n, decades):
             e.append(float(np.sqrt(np.sum(d * d) / np.sum(want * want))))
     ratio = np.log(np.array(here) / np.array(scalar))
     assert ratio.mean() <= 3.0 * ratio.std(ddof=1) / np.sqrt(len(ratio)), (ratio.mean(), ratio.std())
+
+
+@pytest.mark.parametrize("nn,na", [(8, 24), (16, 40), (40, 20)])
+def test_inverse_with_rows_below_is_as_exact_as_a_scalar_one(nn, na):
+    # a front under a root: Y21 = -V W, Y11 = M^T M - Y21^T W with V out of the
+    # root's result; 40 diagonally dominant matrices, compared as above
+    n = nn + na + EXTRA
+    r, c = np.tril_indices(n, -1)
+    keep = (c >= nn) | (r < nn + na)
+    pattern = [grids.spd_from_lower_pattern(n, r[keep], c[keep], seed) for seed in range(40)]
+    s = cp.symbolic(pattern[0])
+    s.plan().set_option("subtrees", 0)
+    here, scalar = [], []
+    for A in pattern:
+        X = cp.cspmatrix(s) + A
+        cp.cholesky(X)
+        B = X.blkval.cpu().numpy()[:(nn + na) * nn].reshape(nn, nn + na).T
+        L, W = np.tril(B[:nn]), B[nn:]
+        cp.projected_inverse(X)
+        Y = X.blkval.cpu().numpy()
+        V = Y[(nn + na) * nn:].reshape(na + EXTRA, na + EXTRA).T[:na, :na]
+        V = np.tril(V) + np.tril(V, -1).T
+        T = np.eye(nn, dtype=np.longdouble)
+        for i in range(nn):
+            T[i] = (T[i] - L[i, :i] @ T[:i]) / L[i, i]
+        want = T.T @ T + W.T.astype(np.longdouble) @ (V.astype(np.longdouble) @ W)
+        S, P = np.zeros((na, nn)), np.zeros((nn, nn))
+        for k in range(na):
+            S = fma(V[:, k:k + 1], W[k:k + 1], S)
+        for k in range(na):
+            P = fma(-S[k][:, None], W[k][None, :], P)
+        for e, Z in ((here, Y[:(nn + na) * nn].reshape(nn, nn + na).T[:nn]), (scalar, scalar_inverse(L) - P)):
+            d = np.tril(Z) - np.tril(want)
+            e.append(float(np.sqrt(np.sum(d * d))))
+    ratio = np.log(np.array(here) / np.array(scalar))
+    assert ratio.mean() <= 3.0 * ratio.std(ddof=1) / np.sqrt(len(ratio)), (ratio.mean(), ratio.std())
