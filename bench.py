@@ -589,9 +589,12 @@ def autograd_section(dev, side=32, value_sets=16, reps=5, h=1e-6):
     (g1,) = torch.autograd.grad(autograd.logdet_values(x, s).sum(), x, create_graph=True)
     (hv,) = torch.autograd.grad((g1 * u[None, :]).sum(), x)
     second = float((hv[0] * u).sum())
-    Hu = U.copy()
-    ref.hessian(s, Lr, Yr, [Hu], adj=None, factored_updates=True)
-    second_ref = -ref.dot(s, U.copy(), Hu)
+    hvp_error = None
+    if ref.available():  # (the one-core restatement takes a minute)
+        Hu = U.copy()
+        ref.hessian(s, Lr, Yr, [Hu], adj=None, factored_updates=True)
+        second_ref = -ref.dot(s, U.copy(), Hu)
+        hvp_error = abs(second - second_ref) / abs(second_ref)
     memory = autograd_memory(dev, s, x0, reps, g)
     return {"workload": "3-D 7-point grid %d^3 (n=%d), AMD, merge_size_fill(32,32), %d value sets through "
                         "chompack_b200.autograd.logdet_values (torch.autograd.grad)" % (side, s.n, value_sets),
@@ -601,7 +604,7 @@ def autograd_section(dev, side=32, value_sets=16, reps=5, h=1e-6):
                                  "reduction (2 kernels) and the gradient weights (1 kernel)"},
             "gradient_rel_error_vs_reference": abs(gU - want) / abs(want),
             "gradient_fd_rel_error": abs(gU - fd) / abs(fd), "fd_step": h,
-            "hvp_rel_error_vs_reference": abs(second - second_ref) / abs(second_ref),
+            "hvp_rel_error_vs_reference": hvp_error, "errors_against": ref.source(),
             "memory": memory}
 
 

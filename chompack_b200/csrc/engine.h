@@ -33,9 +33,10 @@ constexpr int LDS = TILE + 4;     // padded leading dimension of staged tiles
 constexpr int MAX_BASES = 64;     // base-pointer slots (see Base below)
 // Dynamic shared memory of the persistent kernel (doubles).  GEMM and POTRF
 // tasks need ENGINE_SMEM_BASE_DOUBLES (74 KB); programs with Householder
-// panels launch with ENGINE_SMEM_DOUBLES (112 KB, so that two CTAs still fit
-// an SM: 228 KB, 1 KB reserved per CTA).  The others keep the smaller
-// carve-out, which leaves more L1 for the register spills.
+// panels or solve steps launch with ENGINE_SMEM_DOUBLES (112 KB, so that two
+// CTAs still fit an SM: 228 KB, 1 KB reserved per CTA).  The others keep the
+// smaller carve-out, which leaves more L1 for the copies of the operands
+// (chosen while the base build spilled registers; it no longer does).
 constexpr int ENGINE_SMEM_BASE_DOUBLES = 9472;
 constexpr int ENGINE_SMEM_DOUBLES = 14336;
 // T_TRSV: the largest K, and the leading dimensions of its staged operands
@@ -46,7 +47,13 @@ constexpr int TRSV_LA = TILE + 2;
 constexpr int TRSV_LB = TRSV_KMAX + 4;
 static_assert(TRSV_KMAX * TRSV_LA + 8 * TRSV_LB <= ENGINE_SMEM_DOUBLES, "T_TRSV staging exceeds shared memory");
 // Householder panels of h rows.  Up to QL_REG_ROWS rows a panel is reduced in
-// registers, at most 64 entries a thread, which bounds its columns.
+// registers, at most 64 entries a thread, which bounds its columns.  Taller
+// ones are reduced in shared memory, 16 columns at most, where the shared
+// memory alone would allow up to about 25: with 24 factored completion took
+// 63.9 ms against 63.3 on 3-D 40^3, 147.0 / 146.4 on 48^3 and 286.2 / 286.1
+// on 56^3.  A panel may grow past QL_REG_ROWS rows: with growth stopped there
+// 66.8, 147.9 and 288.8 ms.  (All panels in shared memory with seven barriers
+// a reflection: 88.7, 201.9 and 360.5.)
 constexpr int QL_REG_ROWS = 512;
 CHB_HD constexpr int ql_max_cols(int h) { return h <= 128 ? 56 : h <= 256 ? 32 : h <= QL_REG_ROWS ? 12 : 16; }
 // Shared-memory doubles of a panel: the panel (leading dimension ql_ld:

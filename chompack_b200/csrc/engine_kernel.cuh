@@ -1792,7 +1792,7 @@ static __device__ void run_asm(const RunArgs& ra, const Task& t, double* smem) {
 //   5. the block and the update matrix (operand c) written back.
 // A non-positive pivot records ctl[2] = j + 1 and continues with 1.
 // Bound by its chain of steps: with a barrier a pivot and scalar updates a
-// front of 2-D 30^2 (merged) took 34.2 us, in blocks 13.7.
+// front of 2-D 30^2 (merged) took 34.2 us, in blocks 11.4.
 // (Substitution, not products with the inverses of the blocks: those leave a
 // residual that grows with the block's condition, 7e-15 at 4e3.)
 constexpr int FRONT_LD = TILE + 20;             // up to 80 rows; 4 mod 16
@@ -2092,7 +2092,7 @@ __device__ __forceinline__ void warp_mma_any(double (&acc)[4], const double* pa,
 //   the block <- [Y11 (strict upper part zeroed); S21].
 // A zero diagonal entry records ctl[2] = j + 1 and is taken as 1.
 // With scalar dots, two barriers a column of M, a front of 2-D 30^2 (merged)
-// took 24.1 us, now 12.0.
+// took 24.1 us, now 10.1.
 constexpr int PF_LD = TILE + 4;
 static_assert(2 * TILE * PF_LD + TILE + TILE / 2 + 8 <= ENGINE_SMEM_BASE_DOUBLES,
               "small fronts exceed the engine's shared memory");
@@ -2756,10 +2756,12 @@ __device__ __forceinline__ void ql_t_factor(const QlSmem& s) {
 //      T(i+1:, i) = -tau_i T(i+1:, i+1:) W'(:, i+1:)^T w'_i).
 // A panel is a serial chain of reflections: their latency bounds it.  Up to
 // 512 rows it is held in registers (56 columns of 128 rows, 32 of 256, 12 of
-// 512: one slot more spills, and a spilled register costs an L2 round trip
-// with the shared memory of two panels on an SM); taller ones stay in shared
-// memory.  With every panel in shared memory and seven barriers a
-// reflection, a reflection took 4.9k cycles; now 1.7k (128 rows) to 3.0k.
+// 512).  The build spills 40 bytes a thread with these sizes; with 80 entries
+// a thread instead of 64 factored completion on 3-D 40^3 took 70 ms instead
+// of 63, as a spilled register costs an L2 round trip where two panels take an
+// SM's shared memory.  Taller panels stay in shared memory.  With every panel
+// in shared memory and seven barriers a reflection, a reflection took 4.9k
+// cycles; now 1.7k (128 rows) to 3.0k.
 static __device__ void run_ql(const RunArgs& ra, const Task& t, double* smem) {
   const FrontDesc ch = ra.fronts[t.aux[0]];
   const FrontDesc f = ra.fronts[ch.parent];
@@ -3052,7 +3054,7 @@ __device__ __forceinline__ int bundle_last(const Task& t, int w) {
 // Global loads go SUB_E at a time into registers before they are stored (a
 // load is not moved above a store to shared memory, so one by one each costs
 // a round trip: a bundle of the 256 uneven grids took 72 us in cholesky and
-// 67 in projected_inverse, now 55 and 63).
+// 67 in projected_inverse, now 60 and 63).
 constexpr int SUB_E = 8;
 
 // Columns [c0, c1) of a matrix whose column c begins at src + c * ld, rows

@@ -165,7 +165,8 @@ Program* build_host_program(chb_plan* plan, int op, int64_t k, int flags) {
   // and on 2-D 60^2 0.58 / 0.88, factored 62.6 / 68.7 and 2.5 / 3.0, full
   // hessian (unfactored) 31.9 / 35.7 and 1.8 / 2.9, projected_inverse 5.5 /
   // 5.7 and 0.95 / 1.01, on 2-D 1000^2 9.7 / 12.3, and under a scratch limit
-  // 10.8 / 13.7; no sweep at any measured size was faster dynamically.
+  // 10.8 / 13.7; no measured sweep on device-resident values was faster
+  // dynamically.
   // Sweeps on host-resident values run dynamically: a CTA in list order
   // waits on a chunk of the values that has not arrived, while tasks of
   // those that have are ready.  Static against dynamic, cholesky and
@@ -345,8 +346,6 @@ int run_program(chb_plan* plan, Program* prog, void* work, size_t work_bytes, do
 
 using namespace chb;
 
-// Device copies of the plan's symbolic data (skipped with device < 0: a
-// host-only plan for introspection) and the persistent grid size.
 // The pieces of the block values: at most RED_PIECE entries each, cut at the
 // matrices of a merged plan.
 static std::vector<RedPiece> red_pieces(chb_plan* P) {
@@ -368,6 +367,8 @@ static std::vector<RedPiece> red_pieces(chb_plan* P) {
   return v;
 }
 
+// Device copies of the plan's symbolic data (skipped with device < 0: a
+// host-only plan for introspection) and the persistent grid size.
 static int upload_plan(chb_plan* P) {
   const int device = P->device;
   const std::vector<RedPiece> red = red_pieces(P);
