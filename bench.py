@@ -917,7 +917,7 @@ def main():
                 parity["e2e_projected_inverse"] = workload.block_errors(s, Y_e2e, Yr)
             parity["max_scaled_error"] = max(v for k, v in parity.items() if isinstance(v, float) and k != "rtol")
             parity["pass"] = parity["max_scaled_error"] <= RTOL
-        except Exception as exc:  # the checker is reported, never required
+        except Exception as exc:  # the oracle is reported, never required
             parity = {"unavailable": str(exc)}
         peak = fp64_peak_tflops(dev)
         alg_bytes = sweep_bytes(s)

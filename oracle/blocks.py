@@ -1,6 +1,6 @@
 """numpy restatements of the reference's element-wise cspmatrix updates
 (Python loops over supernodes in the reference).  TEST INFRASTRUCTURE ONLY:
-the checker used by tests/, never by the product.
+the oracle used by tests/, never by the product.
 
 `symb` carries the reference's symbolic attributes; `blkval` is a float64
 numpy array in the reference's block layout, updated in place.

@@ -1,5 +1,5 @@
 """numpy restatements of the reference's positive semidefinite completions
-(Python-only in the reference).  TEST INFRASTRUCTURE ONLY: the checker used
+(Python-only in the reference).  TEST INFRASTRUCTURE ONLY: the oracle used
 by tests/, never by the product.
 
 `symb` carries the reference's symbolic attributes; `X0` is the dense

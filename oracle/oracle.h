@@ -1,7 +1,7 @@
 /*
  * Oracle: a plain-C restatement of the reference's numeric multifrontal
  * sweeps (chompack src/C/*.c), with its own naive dense kernels in place of
- * BLAS/LAPACK.  TEST INFRASTRUCTURE ONLY — the checker used by tests/,
+ * BLAS/LAPACK.  TEST INFRASTRUCTURE ONLY — the oracle used by tests/,
  * __graft_entry__.smoke() and bench.py's CPU-baseline leg; never linked into
  * or called by the product.
  *

@@ -1,6 +1,6 @@
 """ctypes driver of oracle/liboracle.so, our plain-C restatement of the
 reference's numeric sweeps (oracle/oracle.c).  TEST INFRASTRUCTURE ONLY: the
-checker used by tests/, never by the product.  Same calling convention as
+oracle used by tests/, never by the product.  Same calling convention as
 oracle/ref.py (numpy arrays; `symb` with the reference's attributes)."""
 import ctypes
 import os

@@ -1,7 +1,7 @@
 """ctypes driver of the reference's own numeric C kernels, compiled unchanged
 into oracle/_ref/libchompack_ref.so by oracle/Makefile.
 
-TEST INFRASTRUCTURE (the checker): only tests/, __graft_entry__.smoke() and
+TEST INFRASTRUCTURE (the oracle): only tests/, __graft_entry__.smoke() and
 bench.py's CPU-baseline / reference legs use this module.  It marshals the
 symbolic arrays and workspaces exactly as the reference's CPython wrapper
 does (src/C/cbase.c: cchol :187-284, cllt :298-390, cprojected_inverse

@@ -1,6 +1,6 @@
 """numpy restatement of the reference's multiplication with the supernodal
 factor (src/python/pybase/trmm.py:4-116, Python only in the reference).
-TEST INFRASTRUCTURE ONLY: the checker used by tests/, never by the product.
+TEST INFRASTRUCTURE ONLY: the oracle used by tests/, never by the product.
 
 `symb` carries the reference's symbolic attributes (snpost, snptr, snode,
 relptr, relidx, chptr, chidx, blkptr, p, n); `blkval` is the factor as the

@@ -1,7 +1,7 @@
 """Inputs of the benchmark workloads for the reference's own kernels, built
 without the product library.
 
-TEST INFRASTRUCTURE (the checker's side): used by bench.py's reference and
+TEST INFRASTRUCTURE (the oracle's side): used by bench.py's reference and
 CPU-baseline legs and by tests/.  Nothing in chompack_b200 imports it, and it
 imports nothing from chompack_b200, so a process that runs only the reference
 kernels (oracle/_ref) maps no library of the product.

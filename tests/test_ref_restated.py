@@ -1,4 +1,4 @@
-"""The checker without the reference's kernels: every function of oracle/ref.py
+"""The oracle without the reference's kernels: every function of oracle/ref.py
 answers from the C restatement, and the restated product form satisfies its
 definition."""
 import numpy as np
