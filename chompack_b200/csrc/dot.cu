@@ -22,31 +22,51 @@ __device__ double block_sum(double v, double* sh) {
   return sh[0];
 }
 
-// The block values in pieces of RED_PIECE consecutive entries (of one
-// matrix; RedPiece, listed once per plan), one CTA per piece and RED_PIECE /
-// 8 entries per warp.  A warp finds the supernode of its first entry by a
-// search between the piece's first supernode and the next piece's, then
-// walks the supernodes, one 64-bit division per supernode to place itself
-// and 32-bit ones per entry.  f(position, row, column) sees every entry
-// once.  Bound by HBM: with one CTA per supernode the largest block (62 MB
-// on a 3-D grid of 40^3) went through one SM with a 64-bit division per
-// entry.  Calls on that grid (30.7 M entries), before and after: dot
-// 11.34 -> 0.118 ms, sym_weight 16.26 -> 0.103 ms (HBM floor 0.075).
-constexpr int RED_WARP = RED_PIECE / (DOT_THREADS / 32);
+// The block values in pieces of consecutive entries (of one matrix; RedPiece,
+// listed once per plan), one CTA per piece and an eighth of its entries per
+// warp.  Where a piece holds few supernodes for its length (RED_FEW entries
+// each, or more) a warp finds the supernode of its first entry by a search
+// between the piece's first supernode and the next piece's, then walks the
+// supernodes, one 64-bit division per supernode to place itself and 32-bit
+// ones per entry; otherwise every entry is searched for, as a walk is a chain
+// of loads per supernode.  f(position, row, column) sees every entry once.
+// Bound by HBM, small plans by the chain of loads: 2-D 10^2 with 80 supernodes
+// in one piece walked by two warps 95 us a dot, now 47, one CTA per supernode
+// 46; unmerged 300^2 98, now 85, and 283.  With one CTA per supernode
+// the largest block (62 MB on a 3-D grid of 40^3) went through one SM with a
+// 64-bit division per entry.  Calls on that grid (30.7 M entries), before and
+// after: dot 11.34 -> 0.118 ms, sym_weight 16.26 -> 0.103 ms (HBM floor 0.075).
+constexpr int RED_FEW = 64;
 template <class F>
 __device__ __forceinline__ void for_entries(const FrontDesc* __restrict__ fronts, const RedPiece* __restrict__ pieces,
                                             int i, F f) {
   const RedPiece p = pieces[i];
-  const int lane = threadIdx.x & 31;
-  const int64_t lo = p.off + (threadIdx.x >> 5) * RED_WARP, hi = min(p.off + p.len, lo + RED_WARP);
+  const int lane = threadIdx.x & 31, share = (p.len + DOT_THREADS - 1) / DOT_THREADS * 32;
+  const int64_t lo = p.off + (threadIdx.x >> 5) * share, hi = min(p.off + p.len, lo + share);
   if (lo >= hi) return;
-  // the last supernode of [p.sn, next piece's] that starts at or before lo
-  int k = p.sn, top = pieces[i + 1].sn;
-  while (k < top) {
-    const int mid = (k + top + 1) >> 1;
-    if (fronts[mid].blk <= lo) k = mid;
-    else top = mid - 1;
+  // the last supernode of [p.sn, next piece's] that starts at or before an entry
+  const int after = pieces[i + 1].sn;
+  auto find = [&](int64_t at) {
+    int k = p.sn, top = after;
+    while (k < top) {
+      const int mid = (k + top + 1) >> 1;
+      if (fronts[mid].blk <= at) k = mid;
+      else top = mid - 1;
+    }
+    return k;
+  };
+  if (p.len < RED_FEW * (after - p.sn)) {
+#pragma unroll 4
+    for (int64_t at = lo + lane; at < hi; at += 32) {
+      const int k = find(at);
+      const int64_t off = at - fronts[k].blk;
+      const unsigned nj = (unsigned)fronts[k].nj;
+      const int64_t c = off >> 32 ? off / nj : (unsigned)off / nj;
+      f(at, (int)(off - c * nj), (int)c);
+    }
+    return;
   }
+  int k = find(lo);
   for (int64_t at = lo; at < hi; k++) {
     const int64_t blk = fronts[k].blk;
     const unsigned nj = (unsigned)fronts[k].nj;
@@ -104,8 +124,10 @@ __global__ void __launch_bounds__(DOT_THREADS) logdet_blocks(const double* __res
 // y = alpha * w .* x over the stored entries, w = 2 below the diagonal, 1 on
 // it, 0 in the strict upper part of a diagonal block: the map from a
 // chordal symmetric matrix to the gradient of a function of its stored
-// entries (<A, B> = sum w a b).
-__global__ void __launch_bounds__(DOT_THREADS) symw_pieces(const double* x, double* y, double alpha,
+// entries (<A, B> = sum w a b).  (Eight CTAs an SM, 32 registers with a spill
+// of 44 bytes: 119 us on 3-D 40^3 against 134 with the 37 registers that do
+// not spill.)
+__global__ void __launch_bounds__(DOT_THREADS, 8) symw_pieces(const double* x, double* y, double alpha,
                                                            const FrontDesc* __restrict__ fronts,
                                                            const RedPiece* __restrict__ pieces) {
   for_entries(fronts, pieces, blockIdx.x, [&](int64_t at, int r, int c) {

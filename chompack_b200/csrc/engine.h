@@ -195,7 +195,16 @@ struct RedPiece {
   int32_t sn;
   int32_t len;
 };
-constexpr int RED_PIECE = 4096;  // entries of a full piece
+// Entries of a full piece: 4096, fewer (a multiple of the 256 threads of a
+// CTA) while that would leave fewer than RED_PIECES pieces.  dot on the 2-D
+// grids 10^2, 100^2 (unmerged) and 300^2 (merge 16), us: pieces of 4096 always
+// 95, 95, 62; 296 pieces 48, 49, 64; 1024 47, 50, 64; 2048 46, 49, 70.
+constexpr int RED_PIECE = 4096, RED_PIECE_MIN = 256, RED_PIECES = 1024;
+CHB_HD constexpr int64_t red_piece(int64_t total) {
+  return total >= (int64_t)RED_PIECE * RED_PIECES ? RED_PIECE
+         : total <= (int64_t)RED_PIECE_MIN * RED_PIECES ? RED_PIECE_MIN
+                                                        : total / RED_PIECES / RED_PIECE_MIN * RED_PIECE_MIN;
+}
 
 // Device-side run description (passed by value to the persistent kernel).
 struct RunArgs {

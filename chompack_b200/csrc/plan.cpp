@@ -346,19 +346,20 @@ int run_program(chb_plan* plan, Program* prog, void* work, size_t work_bytes, do
 
 using namespace chb;
 
-// The pieces of the block values: at most RED_PIECE entries each, cut at the
+// The pieces of the block values: at most red_piece() entries each, cut at the
 // matrices of a merged plan.
 static std::vector<RedPiece> red_pieces(chb_plan* P) {
   std::vector<RedPiece> v;
+  const int64_t full = red_piece(P->blk_total);
   P->red_seg.assign(1, 0);
   for (size_t m = 0; m + 1 < P->seg.size(); m++) {
     const int64_t k0 = P->seg[m], k1 = P->seg[m + 1];
     const int64_t beg = k0 < P->nsn ? P->fronts[k0].blk : P->blk_total;
     const int64_t end = k1 < P->nsn ? P->fronts[k1].blk : P->blk_total;
     int64_t k = k0;
-    for (int64_t o = beg; o < end; o += RED_PIECE) {
+    for (int64_t o = beg; o < end; o += full) {
       while (k + 1 < k1 && P->fronts[k + 1].blk <= o) k++;
-      v.push_back({o, (int32_t)k, (int32_t)std::min<int64_t>(RED_PIECE, end - o)});
+      v.push_back({o, (int32_t)k, (int32_t)std::min<int64_t>(full, end - o)});
     }
     P->red_seg.push_back((int64_t)v.size());
   }
