@@ -2852,6 +2852,48 @@ static __device__ void run_ql(const RunArgs& ra, const Task& t, double* smem) {
 }
 
 // ------------------------------------------------------- solve vectors
+// Extraction of a child's rows out of [x_p; u_p], or (add) their addition into
+// it: elements idx < tot, row i0 + idx mod ni of u_c, column j0 + idx / ni,
+// EV per thread at a time.
+struct VecChild {
+  const int32_t* r;  // relative indices of the child
+  double *uc, *xp, *up;
+  int nn, na, Nc, ldx, i0, ni, j0, tot;
+};
+template <int EV>
+__device__ __forceinline__ void vec_child(const VecChild& a, bool add) {
+  for (int base = 0; base < a.tot; base += EV * NTHREADS) {
+    int row[EV], col[EV];
+    double v[EV];
+#pragma unroll
+    for (int e = 0; e < EV; e++) {
+      const int idx = base + threadIdx.x + e * NTHREADS;
+      const int j = idx / max(a.ni, 1), i = a.i0 + idx - j * a.ni;
+      col[e] = a.j0 + j;
+      row[e] = (idx < a.tot) ? __ldg(a.r + i) : -1;
+      if (add) v[e] = (idx < a.tot) ? __ldcg(a.uc + i + (int64_t)(a.j0 + j) * a.Nc) : 0.0;
+    }
+    auto entry = [&](int e) {
+      return row[e] < a.nn ? a.xp + row[e] + (int64_t)col[e] * a.ldx : a.up + (row[e] - a.nn) + (int64_t)col[e] * a.na;
+    };
+    if (add) {
+      // rows of one child are distinct, but other children add into the
+      // same rows at the same time: atomic adds
+#pragma unroll
+      for (int e = 0; e < EV; e++)
+        if (row[e] >= 0) atomicAdd(entry(e), v[e]);
+      continue;
+    }
+#pragma unroll
+    for (int e = 0; e < EV; e++) v[e] = row[e] < 0 ? 0.0 : __ldcg(entry(e));
+#pragma unroll
+    for (int e = 0; e < EV; e++) {
+      const int idx = base + threadIdx.x + e * NTHREADS;
+      if (row[e] >= 0) a.uc[a.i0 + idx - (col[e] - a.j0) * a.ni + (int64_t)col[e] * a.Nc] = v[e];
+    }
+  }
+}
+
 // Vector operations of the triangular solve sweep (T_VEC, sub-operation
 // aux[0], nrhs = t.n right-hand sides).  Bp / x_k live at operand a or c
 // with leading dimension n; the per-front vector updates u_k (na x nrhs,
@@ -2997,40 +3039,14 @@ static __device__ void run_vec(const RunArgs& ra, const Task& t, double* smem) {
   const int i0 = t.m, i1 = t.k > 0 ? t.k : Nc, ni = max(i1 - i0, 0), tot = ni * nc;
   const int32_t* __restrict__ r = ra.relidx + ch.relptr;
   double* __restrict__ uc = WS + vbase + ch.vpos * nrhs;
-  // EV elements per thread with their loads in flight together: the planner's
+  // 16 elements per thread with their loads in flight together: the planner's
   // chunks (2048 elements) take one pass, two L2 round trips in an extraction
-  // and one in an addition, whose values need not wait for the indices
-  constexpr int EV = 16;
-  for (int base = 0; base < tot; base += EV * NTHREADS) {
-    int row[EV], col[EV];
-    double v[EV];
-#pragma unroll
-    for (int e = 0; e < EV; e++) {
-      const int idx = base + threadIdx.x + e * NTHREADS;
-      const int j = idx / max(ni, 1), i = i0 + idx - j * ni;
-      col[e] = j0 + j;
-      row[e] = (idx < tot) ? __ldg(r + i) : -1;
-      if (mode == VEC_ADD) v[e] = (idx < tot) ? __ldcg(uc + i + (int64_t)(j0 + j) * Nc) : 0.0;
-    }
-    auto entry = [&](int e) {
-      return row[e] < f.nn ? xp + row[e] + (int64_t)col[e] * ldx : up + (row[e] - f.nn) + (int64_t)col[e] * f.na;
-    };
-    if (mode == VEC_ADD) {
-      // rows of one child are distinct, but other children add into the
-      // same rows at the same time: atomic adds
-#pragma unroll
-      for (int e = 0; e < EV; e++)
-        if (row[e] >= 0) atomicAdd(entry(e), v[e]);
-      continue;
-    }
-#pragma unroll
-    for (int e = 0; e < EV; e++) v[e] = row[e] < 0 ? 0.0 : __ldcg(entry(e));
-#pragma unroll
-    for (int e = 0; e < EV; e++) {
-      const int idx = base + threadIdx.x + e * NTHREADS;
-      if (row[e] >= 0) uc[i0 + idx - (col[e] - j0) * ni + (int64_t)col[e] * Nc] = v[e];
-    }
-  }
+  // and one in an addition, whose values need not wait for the indices; at
+  // most 512 elements take four (twelve empty ones are a microsecond: an
+  // extraction on small fronts 2.5 us instead of 1.5).
+  const VecChild c{r, uc, xp, up, f.nn, f.na, Nc, ldx, i0, ni, j0, tot};
+  if (tot <= 4 * NTHREADS) vec_child<4>(c, mode == VEC_ADD);
+  else vec_child<16>(c, mode == VEC_ADD);
 }
 
 // ---------------------------------------------------------------- kernel
