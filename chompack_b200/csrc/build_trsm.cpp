@@ -59,8 +59,13 @@ int build_trsm(const chb_plan& P, Program& prog, int64_t nrhs, bool trans, bool 
   // columns with zeros, a pair of 40^3 solves took 1.45 ms instead of 1.66
   // with 16 right-hand sides and 2.22 instead of 2.26 with 32, but 3.84
   // instead of 3.65 with 64, where the tiles' MMAs reuse their operands.
+  // Short products ('N', K < 64) of more than 24 right-hand sides are tiles
+  // too: four groups of columns are four round trips, a tile's ring one; 32
+  // on 2-D 50^2 with extra neighbours 425 us against 463, on 10^2 190 against
+  // 202 (with 24 191 and 193).  'T' gains from narrow ones throughout (475
+  // against 552).
   auto narrow = [&](Task& t) {
-    if (t.n <= 32 && t.k <= TRSV_KMAX) t.aux[0] = GEMM_NARROW;
+    if (t.n <= (trans || t.k >= 64 ? 32 : 24) && t.k <= TRSV_KMAX) t.aux[0] = GEMM_NARROW;
   };
 
   // workspace: Bp (n x nrhs, ld n); u_k (na x nrhs, ld na) per front; per
