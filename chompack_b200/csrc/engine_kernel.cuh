@@ -933,7 +933,7 @@ static __device__ void store_acc(double* __restrict__ C, int ldc, int m, int n, 
 //   pass 1: D -= L L^T (lower part), L read back from L2
 // Both passes share one inlined copy of the GEMM code: a second copy (or a
 // call) makes the persistent kernel spill.
-template <bool TC>
+template <bool TC, bool EARLY>
 __device__ void run_gemm_or_la(const RunArgs& ra, const Task& t, const SmemLayout& sm, TcState& ts, int& claim) {
   const bool la = t.op == T_LA;
   const int passes = la ? 2 : 1;
@@ -954,8 +954,8 @@ __device__ void run_gemm_or_la(const RunArgs& ra, const Task& t, const SmemLayou
     if (la || t.c.prec == PREC_FP64) gemm_acc_p<PREC_FP64>(A, B, m, n, K, sm, acc);
     else if (t.c.prec == PREC_TF32) gemm_acc_p<PREC_TF32>(A, B, m, n, K, sm, acc);
     else gemm_acc_p<PREC_TF32X3>(A, B, m, n, K, sm, acc);
-    // static: claim the next task, whose index comes back during the epilogue
-    if (!ra.dynamic && ph == passes - 1 && threadIdx.x == 32) claim = atomicAdd(&ra.ctl[0], 1);
+    // static, EARLY: claim the next task, whose index comes back during the epilogue
+    if (EARLY && !ra.dynamic && ph == passes - 1 && threadIdx.x == 32) claim = atomicAdd(&ra.ctl[0], 1);
     if (!la && t.cmode == CM_ATOMIC) store_acc_atomic(ra.bases[oc.base] + oc.off, oc.ld, m, n, alpha, acc);
     else store_acc(ra.bases[oc.base] + oc.off, oc.ld, m, n, lower, cdiag, alpha, beta, acc);
     if (la && ph == 0) {
@@ -3272,6 +3272,7 @@ static_assert(8 * SUB_NJ * SUB_LD <= ENGINE_SMEM_BASE_DOUBLES, "bundle fronts ex
 template <int BUILD>
 __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
   constexpr bool TC = BUILD == EB_TCGEN05;
+  constexpr bool LATE = BUILD == EB_SOLVE;
   constexpr bool FRONTS = BUILD == EB_BASE || TC;  // small fronts and bundles (cholesky, projected_inverse)
   extern __shared__ __align__(16) double smem[];
   __shared__ int s_task;
@@ -3411,7 +3412,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
     claim = -1;
     switch (is_narrow<BUILD>(t) ? T_TRSV : t.op) {
       case T_GEMM:
-      case T_LA: run_gemm_or_la<TC>(ra, t, sm, ts, claim); break;
+      case T_LA: run_gemm_or_la<TC, !LATE>(ra, t, sm, ts, claim); break;
       case T_MROW: run_mrow(ra, t, sm); break;
       case T_POTRF: run_potrf(ra, t, smem, ti); break;
       case T_ASM: run_asm(ra, t, smem); break;
@@ -3458,9 +3459,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) engine_kernel(RunArgs ra) {
     // static: the next task is claimed before this one's end is published,
     // so that its record and waits are fetched (warp 1) beside the release
     // (warp 0).  Its holder still publishes first, whatever the claimed task
-    // waits on.
-    if (!ra.dynamic && threadIdx.x == 32 && claim < 0) claim = atomicAdd(&ra.ctl[0], 1);
+    // waits on.  LATE: beside the release, since in a chain of products, which
+    // has idle CTAs enough, a claim before it delays the end: a product with
+    // the factor of 3-D 40^3 ('N', one column) took 8.11 ms, now 7.95, with
+    // a dense one of order 1500 2.51, now 2.44.
+    if (!LATE && !ra.dynamic && threadIdx.x == 32 && claim < 0) claim = atomicAdd(&ra.ctl[0], 1);
     __syncthreads();
+    if (LATE && !ra.dynamic && threadIdx.x == 32 && claim < 0) claim = atomicAdd(&ra.ctl[0], 1);
     if (threadIdx.x == 0 && ra.trace) {
       ra.trace[4 * (int64_t)ti + 2] = global_ns();
       ra.trace[4 * (int64_t)ti + 3] = (unsigned long long)sm_id() | ((unsigned long long)op << 32);
