@@ -7,7 +7,8 @@
 // reach their targets (bounded spin; on timeout the CTA records DE_TIMEOUT
 // and leaves, so a planning error can never hang the GPU), executes the task,
 // then publishes its counter with release semantics; the claim of the next
-// task goes out before that, in a GEMM task during its epilogue.  Dynamic: a
+// task goes out before that, in a GEMM task during its epilogue (in the build
+// of the solves and products beside the release).  Dynamic: a
 // finished task releases its waiters itself and keeps one of them; idle CTAs
 // claim the others from a ready bitmap (bounded polling, same timeout rule).
 //

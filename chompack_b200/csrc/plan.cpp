@@ -171,7 +171,9 @@ Program* build_host_program(chb_plan* plan, int op, int64_t k, int flags) {
   // waits on a chunk of the values that has not arrived, while tasks of
   // those that have are ready.  Static against dynamic, cholesky and
   // projected_inverse on 3-D 40^3 18.5 / 13.8 and 18.1 / 13.9 ms, on 24^3 2.11
-  // / 2.06 and 2.42 / 2.05, on 2-D 400^2 9.1 / 7.0 and 9.4 / 6.8.
+  // / 2.06 and 2.42 / 2.05, on 2-D 400^2 9.1 / 7.0 and 9.4 / 6.8; small ones
+  // lose up to 0.2 ms by it (pinned, 2-D 100^2 1.07 / 1.16 and 0.71 / 0.88, 3-D
+  // 16^3 0.96 / 0.90 and 0.60 / 0.72).
   prog->static_default = !prog->io.in && !prog->io.out;
   Program* p = prog.get();
   plan->progs[key] = std::move(prog);
